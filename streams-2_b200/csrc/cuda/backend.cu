@@ -234,11 +234,23 @@ void fill_geom(streams_b200_ctx* c) {
   g.gm1 = g.gamloc - 1.0;
   g.rgm1 = 1.0 / g.gm1;
   {
-    // the same products and quotients the reference forms in wenorec_1d (u0_2, rho0_2u0_2, ...)
-    const double u0_2 = p.u0 * p.u0, r2u2 = p.rho0 * p.rho0 * u0_2, r2u4 = r2u2 * u0_2;
-    g.wbs_a = 1.0 / r2u2;
-    g.wbs_b = 1.0 / r2u4;
-    g.wbs_c = g.wbs_b / u0_2;
+    // the same products the reference forms in wenorec_1d (u0_2, rho0_2u0_2, ...)
+    const double u0_2 = p.u0 * p.u0, r2u2 = p.rho0 * p.rho0 * u0_2, r2u4 = r2u2 * u0_2, r2u6 = r2u4 * u0_2;
+    g.rcp0 = 1.0 / p.cp0;
+    g.weps_a = 0.000001 * r2u2;
+    g.weps_b = 0.000001 * r2u4;
+    g.weps_c = 0.000001 * r2u6;
+    auto pow2 = [](double v) { return std::exp2(std::round(std::log2(v > 0.0 && std::isfinite(v) ? v : 1.0))); };
+    g.wsg_a = pow2(1.0 / std::sqrt(r2u2));
+    g.wsg_b = pow2(1.0 / std::sqrt(r2u4));
+    g.wsg_c = pow2(1.0 / std::sqrt(r2u6));
+    g.wsg_ai = 1.0 / g.wsg_a;
+    g.wsg_bi = 1.0 / g.wsg_b;
+    g.wsg_ci = 1.0 / g.wsg_c;
+    g.wepsf_a = g.weps_a * g.wsg_a * g.wsg_a;
+    g.wepsf_b = g.weps_b * g.wsg_b * g.wsg_b;
+    g.wepsf_c = g.weps_c * g.wsg_c * g.wsg_c;
+    g.wepsf_ab = g.weps_b * g.wsg_a * g.wsg_a;
   }
   g.calorically_perfect = p.calorically_perfect;
   g.cp_l = p.indx_cp_l;

@@ -109,7 +109,7 @@ template <unsigned SPAN, class R, int LB, int WS, int FS>
 __global__ void __launch_bounds__(XF_NT, sizeof(R) == 8 ? XF_MINB_D : XF_MINB_F)
     kb_xflux(const BoxRec* __restrict__ rec, const BlockRef* __restrict__ blocks, unsigned ntile, int istep) {
   for_tiles<SPAN>(rec, blocks, ntile, [&](const BoxRec* r, const Geom& g, unsigned l) {
-    d_xflux<R, LB, WS, FS>(g, static_cast<const R*>(r->aux), r->sensor, fl_new_of(r, istep), Blk{l, 0, 0});
+    d_xflux<R, LB, WS, FS>(g, static_cast<const R*>(r->aux), r->sensor, fl_new_of(r, istep), r->xgrp, Blk{l, 0, 0});
   });
 }
 
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(256) kb_sensor(const BoxRec* __restrict__ rec,
 }
 
 template <unsigned SPAN, class R, int DIR, int LB, int WS, bool CH, int FS>
-__global__ void __launch_bounds__(MT_NT, sizeof(R) == 8 ? MT_MINB_D : (CH ? MT_MINB_F_CH : MT_MINB_F))
+__global__ void __launch_bounds__(sizeof(R) == 8 ? MT_MAXT_D : MT_MAXT_F, 1)
     kb_march(const BoxRec* __restrict__ rec, const BlockRef* __restrict__ blocks, unsigned ntile, double rhork, double gamrk, int istep) {
   for_tiles<SPAN>(rec, blocks, ntile, [&](const BoxRec* r, const Geom& g, unsigned l) {
     const int seglen = DIR == 1 ? r->sly : r->slz, nseg = DIR == 1 ? r->nsy : r->nsz;
@@ -242,20 +242,18 @@ cudaError_t batch_stage_impl(const BoxTable& t, const StageArgs& a, cudaStream_t
   constexpr bool TP = (FS & 2) != 0;
   const int nbox = t.nbox;
   if (a.run_aux) batch_aux<R>(t, a.apply_shift, !fp64 && a.istep == 3, s, nl);
-  const size_t xsm = weno_scratch_bytes<R, WS>(XF_NT);
-  const size_t msm = weno_scratch_bytes<R, WS>(MT_NT);
   static unsigned long long smem_set = 0;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !(smem_set & (1ULL << dev))) {
-    cudaFuncSetAttribute(kb_xflux<1, R, LB, WS, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xsm);
-    cudaFuncSetAttribute(kb_march<1, R, 1, LB, WS, false, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm);
-    cudaFuncSetAttribute(kb_march<1, R, 2, LB, WS, false, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm);
-    cudaFuncSetAttribute(kb_march<1, R, 2, LB, WS, true, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm);
+    cudaFuncSetAttribute(kb_xflux<1, R, LB, WS, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, X_SMEM_MAX);
+    for (auto fn : {(const void*)kb_march<1, R, 1, LB, WS, false, FS>, (const void*)kb_march<1, R, 2, LB, WS, false, FS>,
+                    (const void*)kb_march<1, R, 2, LB, WS, true, FS>})
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, MARCH_SMEM_MAX);
     smem_set |= 1ULL << dev;
   }
-  const Launch X = launch_of(t, BK_X), P = launch_of(t, BK_PT), Y = launch_of(t, BK_Y), Z = launch_of(t, BK_Z);
-  kb_xflux<1, R, LB, WS, FS><<<X.grid(1), dim3(XF_TX, XF_TY), xsm, s>>>(t.rec, X.blocks, X.ntile, a.istep);
+  const Launch X = launch_of(t, BK_X), P = launch_of(t, BK_PT);
+  kb_xflux<1, R, LB, WS, FS><<<X.grid(1), dim3(XF_TX, XF_TY), XF_TY * x_warp_bytes<R, WS>(t.xslots), s>>>(t.rec, X.blocks, X.ntile, a.istep);
   const int do_sensor = fp64 && a.istep == 3;
   if (g.conservative_viscous && SB_VISC_TILED) {
     const Launch V = launch_of(t, BK_VS);
@@ -269,19 +267,23 @@ cudaError_t batch_stage_impl(const BoxTable& t, const StageArgs& a, cudaStream_t
     kb_sensor<SPAN_PT><<<P.grid(SPAN_PT), 256, 0, s>>>(t.rec, P.blocks, P.ntile, a.run_aux);
     ++*nl;
   }
-  if (Y.ntile > 0) {
-    kb_march<1, R, 1, LB, WS, false, FS><<<Y.grid(1), MT_NT, msm, s>>>(t.rec, Y.blocks, Y.ntile, a.rhork, a.gamrk,
-                                                                       a.istep);
+  // the y and z passes: a launch per block size of the group's boxes
+  for (const MarchLaunch& m : t.march[0]) {
+    kb_march<1, R, 1, LB, WS, false, FS><<<m.cnt, 32 * m.nwarps, march_smem<R, LB, WS>(m.nwarps, m.maxseg), s>>>(
+        t.rec, t.blocks + m.off, m.cnt, a.rhork, a.gamrk, a.istep);
+    ++*nl;
+  }
+  for (const MarchLaunch& m : t.march[1]) {
+    if (g.channel_case)
+      kb_march<1, R, 2, LB, WS, true, FS><<<m.cnt, 32 * m.nwarps, march_smem<R, LB, WS>(m.nwarps, m.maxseg), s>>>(
+          t.rec, t.blocks + m.off, m.cnt, a.rhork, a.gamrk, a.istep);
+    else
+      kb_march<1, R, 2, LB, WS, false, FS><<<m.cnt, 32 * m.nwarps, march_smem<R, LB, WS>(m.nwarps, m.maxseg), s>>>(
+          t.rec, t.blocks + m.off, m.cnt, a.rhork, a.gamrk, a.istep);
     ++*nl;
   }
   if (g.channel_case) {
-    kb_march<1, R, 2, LB, WS, true, FS><<<Z.grid(1), MT_NT, msm, s>>>(t.rec, Z.blocks, Z.ntile, a.rhork, a.gamrk,
-                                                                      a.istep);
     kb_finish_rhs<<<nbox, FIN_NT, 0, s>>>(t.rec, a.istep == 1);
-    *nl += 2;
-  } else {
-    kb_march<1, R, 2, LB, WS, false, FS><<<Z.grid(1), MT_NT, msm, s>>>(t.rec, Z.blocks, Z.ntile, a.rhork, a.gamrk,
-                                                                       a.istep);
     ++*nl;
   }
   const Launch U = launch_of(t, BK_UP);
@@ -365,14 +367,15 @@ BoxRec box_rec(const Geom& g, const DevState& d, double* fl_a, double* fl_b, dou
   r.red = d.red;
   r.sc = d.sc;
   r.cfl = cfl;
-  long long nty, ntz;
-  march_split(g, 1, &r.sly, &r.nsy, &nty);
-  march_split(g, 2, &r.slz, &r.nsz, &ntz);
-  r.xg[0] = x_blocks(g);
-  r.xg[1] = 1;
-  r.xg[2] = 1;
-  r.nb_y = nblocks(nty, MT_NT);
-  r.nb_z = nblocks(ntz, MT_NT);
+  const MarchShape my = march_shape(g, 1), mz = march_shape(g, 2);
+  r.sly = my.seglen; r.nsy = my.nseg;
+  r.slz = mz.seglen; r.nsz = mz.nseg;
+  r.nwy = my.nwarps; r.nwz = mz.nwarps;
+  const XShape xs = x_shape(g);
+  r.nb_x = xs.nblk;
+  r.xgrp = xs.ngrp;
+  r.nb_y = my.nblk;
+  r.nb_z = mz.nblk;
   r.nb_pt = nblocks(g.nint, 256);
   r.nb_vol = nblocks(g.nvol, AUX_NT);
   r.nb_vs = visc_tiled_blocks(g);
@@ -396,13 +399,30 @@ cudaError_t box_table_build(BoxTable& t, const std::vector<BoxRec>& recs, cudaSt
   std::vector<BlockRef> blocks;
   for (int k = 0; k < BK_NUM; ++k) {
     t.off[k] = (long long)blocks.size();
+    if (k == BK_Y || k == BK_Z) {  // listed by the block size of the box's own pass
+      auto& list = t.march[k == BK_Y ? 0 : 1];
+      list.clear();
+      for (int nw = 1; nw <= MT_MAXW; ++nw) {
+        MarchLaunch m{nw, 1, (long long)blocks.size(), 0};
+        for (size_t b = 0; b < recs.size(); ++b) {
+          const BoxRec& r = recs[b];
+          if ((k == BK_Y ? r.nwy : r.nwz) != nw) continue;
+          m.maxseg = std::max(m.maxseg, k == BK_Y ? r.sly : r.slz);
+          const unsigned nb = k == BK_Y ? r.nb_y : r.nb_z;
+          for (unsigned q = 0; q < nb; ++q) blocks.push_back(BlockRef{(unsigned)b, q});
+        }
+        const long long c = (long long)blocks.size() - m.off;
+        if (c > 0x7fffffffLL) return cudaErrorInvalidValue;  // one launch's grid
+        m.cnt = (unsigned)c;
+        if (c) list.push_back(m);
+      }
+      continue;
+    }
     for (size_t b = 0; b < recs.size(); ++b) {
       const BoxRec& r = recs[b];
       const unsigned long long n = k == BK_VOL ? r.nb_vol
                                    : k == BK_PT ? r.nb_pt
-                                   : k == BK_X  ? (unsigned long long)r.xg[0] * r.xg[1] * r.xg[2]
-                                   : k == BK_Y  ? r.nb_y
-                                   : k == BK_Z  ? r.nb_z
+                                   : k == BK_X  ? r.nb_x
                                    : k == BK_VS ? r.nb_vs
                                                 : r.nb_up;
       for (unsigned long long q = 0; q < n; ++q) blocks.push_back(BlockRef{(unsigned)b, (unsigned)q});
@@ -424,6 +444,8 @@ cudaError_t box_table_build(BoxTable& t, const std::vector<BoxRec>& recs, cudaSt
   }
   t.nbox = (int)recs.size();
   t.g0 = recs[0].g;
+  t.xslots = 1;
+  for (const BoxRec& r : recs) t.xslots = std::max(t.xslots, x_shape(r.g).slots);
   return cudaSuccess;
 }
 

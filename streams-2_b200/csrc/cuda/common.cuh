@@ -79,10 +79,13 @@ struct Geom {
   int visc_model;
   double mu0, t0, rgas0, rho0, u0, l0, sutherland_s, t_ref_dim, vtexp, prandtl;
   double cp0, cv0, cp_last, cv_last, gamloc;
-  // constants of the WENO faces formed once on the host: gamma - 1 and 1/(gamma - 1) of the
-  // calorically perfect gas, the smoothness-indicator scales 1/(rho0^2 u0^2) and
-  // 1/(rho0^2 u0^4) of wenorec_1d (kernels_cpu.F90:2539-2546) and 1/(rho0^2 u0^6)
-  double gm1, rgm1, wbs_a, wbs_b, wbs_c;
+  // constants of the WENO faces formed once on the host: gamma - 1, 1/(gamma - 1) and 1/cp of the
+  // calorically perfect gas, and the 1e-6 of the weights over the smoothness-indicator scales
+  // 1/(rho0^2 u0^2) and 1/(rho0^2 u0^4) of wenorec_1d (kernels_cpu.F90:2539-2546) and
+  // 1/(rho0^2 u0^6).  FP32 values are scaled by powers of two wsg near the square roots of those
+  // scales (wsg_*i their reciprocals): wepsf = wsg^2 weps, wepsf_ab with the scale b and wsg_a
+  double gm1, rgm1, rcp0, weps_a, weps_b, weps_c;
+  double wsg_a, wsg_b, wsg_c, wsg_ai, wsg_bi, wsg_ci, wepsf_a, wepsf_b, wepsf_c, wepsf_ab;
   // thermally perfect gas (calorically_perfect = 0): cp(T) = sum of cpc[l - cp_l] (T/t0)^l for
   // l = cp_l..cp_r, cv likewise (set_fluid_prop's cp_coeff / cv_coeff, times rgas0)
   int calorically_perfect, cp_l, cp_r;
@@ -96,8 +99,8 @@ struct Geom {
   int precision;
   // WENO faces computed apart from the hybrid passes: per direction the list of the faces whose
   // stencil sees the sensor (rebuilt at stage 1, the sensor being fixed for a step) and one face
-  // buffer of their fluxes (planes of nwface values: 5 in FP64, 5 high + 5 low parts in FP32)
-  void* wface;
+  // buffer of their fluxes (5 planes of nwface FP64 values)
+  double* wface;
   long long nwface;
   unsigned int* wlist[3];
   unsigned int* wcount;  // [3]

@@ -6,20 +6,6 @@
 
 #include "common.cuh"
 
-// keep the sound speed of every stencil point in the window (1) or recompute it in the WENO
-// branch (0, default: fewer registers and spills in the march kernels, measured 2-7 % faster)
-#ifndef SB_CACHE_C
-#define SB_CACHE_C 0
-#endif
-
-// characteristic fields reconstructed per iteration of the WENO branch's field loop (1: one copy
-// of wenorec, the loop rolled; the unrolled loop overflowed the instruction cache)
-#ifndef SB_WENO_UNROLL
-#define SB_WENO_UNROLL 1
-#endif
-#define SB_PRAGMA_(x) _Pragma(#x)
-#define SB_UNROLL_(n) SB_PRAGMA_(unroll n)
-
 // quotients and square roots of the mixed form's FP32 flux arithmetic: IEEE (0), the hardware
 // approximations (1), or the hardware approximations refined by one Newton step (2)
 #ifndef SB_FP32_FAST
@@ -64,261 +50,205 @@ __device__ __forceinline__ R fsqrt_pos(R x) {
   }
 }
 
-// Error-free transformations for the mixed form: the face fluxes are accumulated as float-float
-// pairs (hi + lo) so that the flux differences of neighbouring faces can be formed in FP64
-// without the cancellation of the FP32 rounding of their final sums.  Explicit rounding
-// intrinsics keep the compiler from contracting them.
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-  s = __fadd_rn(a, b);
-  const float bb = __fsub_rn(s, a);
-  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+// Reciprocal and reciprocal square root in the FP64 flux arithmetic: the hardware's approximation y
+// (about 20 correct bits) corrected by the first terms of the binomial series of its residual,
+//   1/b = y/(1 - e) = y (1 + e + e^2 + ..),               e = 1 - b y,
+//   1/sqrt(x) = y/sqrt(1 - e) = y (1 + e/2 + 3 e^2/8 + ..),  e = 1 - x y^2,
+// which leaves e^3 (below 2^-57) and the rounding of the last operations, about one unit in the
+// last place.  Arguments are positive and normal (densities, squared sound speeds, sums of weights).
+// They stand for the IEEE quotients and square roots, which branch for their special cases, of the
+// Roe average (three) and of the weights (one for the two sides of a field) of a WENO face.
+__device__ __forceinline__ double rcp_pos(double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  const double e = fma(-b, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
-// acc (hi, lo) += a * b
-__device__ __forceinline__ void acc_prod(float& hi, float& lo, float a, float b) {
-  const float p = __fmul_rn(a, b);
-  const float ep = __fmaf_rn(a, b, -p);
-  float s, es;
-  two_sum(hi, p, s, es);
-  hi = s;
-  lo = lo + (es + ep);
+__device__ __forceinline__ float rcp_pos(float b) { return fdiv(1.0f, b); }
+__device__ __forceinline__ double rsqrt_pos(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
 }
-__device__ __forceinline__ void acc_prod(double& hi, double& lo, double a, double b) {
-  hi = hi + a * b;
-  (void)lo;
-}
-__device__ __forceinline__ void acc_add(float& hi, float& lo, float b) {
-  float s, es;
-  two_sum(hi, b, s, es);
-  hi = s;
-  lo = lo + es;
-}
-__device__ __forceinline__ void acc_add(double& hi, double& lo, double b) {
-  hi = hi + b;
-  (void)lo;
-}
+__device__ __forceinline__ float rsqrt_pos(float x) { return rsqrt(x); }
+// maximum that keeps b when a is not a number (as fmax does for the running maxima here), without
+// fmax's handling of two of them in FP64
+__device__ __forceinline__ double max_of(double a, double b) { return a > b ? a : b; }
+__device__ __forceinline__ float max_of(float a, float b) { return fmaxf(a, b); }
 
-// 1/a and 1/b from one division in FP64, 1/(a b) times the other factor: the weight sums of
-// the two sides of a WENO reconstruction are positive and stay far inside the FP64 exponent
-// range (products of (eps + beta)^2 terms, eps = 1e-6, or WENO-Z ratios), so the product neither
-// overflows nor underflows.  FP32 keeps two divisions (its range is too narrow for the product).
+// The stencil of a face: point q = 0 .. 2S-1 (offsets -(S-1) .. S from the face's lower point) of
+// field f (rho, u, v, w, H, T and, in the FP64 form, F_C, the sound speed).
+constexpr int F_C = 6;
+// in global memory
 template <class R>
-__device__ __forceinline__ void recip_pair(R a, R b, R& ra, R& rb) {
-  if constexpr (sizeof(R) == sizeof(double)) {
-    const R r = R(1) / (a * b);
-    ra = b * r;
-    rb = a * r;
-  } else {
-    ra = fdiv(R(1), a);
-    rb = fdiv(R(1), b);
+struct Line {
+  const R* p;        // field 0 at point 0
+  long long n, sd;   // strides of the fields and of the points
+  __device__ __forceinline__ R operator()(int f, int q) const { return __ldg(p + (f == F_C ? 7 : f) * n + q * sd); }
+};
+// in a ring of points in shared memory, 32 lanes of a field in a row, RF fields a point.  The reads
+// are volatile: the compiler would otherwise keep the stencil in registers from its first use to
+// its last (36 values in 72 registers), where a second read costs one instruction.
+template <class R>
+constexpr int ring_fields() { return sizeof(R) == sizeof(double) ? 7 : 6; }
+template <class R, int NP>
+struct Ring {
+  unsigned o[NP];    // shared address of this lane's field 0 at point q
+  __device__ __forceinline__ R operator()(int f, int q) const {
+    R v;
+    if constexpr (sizeof(R) == sizeof(double)) asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(o[q] + f * 256));
+    else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(o[q] + f * 128));
+    return v;
   }
-}
+};
 
-// Stencil of a face: NP = 2*S points at offsets o = -(S-1) .. S from the face's lower point.
+// in a row of points in shared memory, XS values a point (an odd count: lanes at consecutive points
+// meet no bank twice), lane by lane from its own first point
+constexpr int XS = 7;
+template <class R>
+struct RowPts {
+  unsigned o;        // shared address of field 0 at point 0
+  __device__ __forceinline__ R operator()(int f, int q) const {
+    R v;
+    if constexpr (sizeof(R) == sizeof(double)) asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(o + (q * XS + f) * 8));
+    else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(o + (q * XS + f) * 4));
+    return v;
+  }
+};
+
+// Stencil of a face in registers: NP = 2*S points.
 template <class R, int S>
 struct Stencil {
   R rho[2 * S], u[2 * S], v[2 * S], w[2 * S], h[2 * S], t[2 * S];
-#if SB_CACHE_C
-  R c[2 * S];  // sound speed sqrt(gamma R T) of each point, computed once when the point is loaded
-#endif
 };
 
-// wenorec_1d (kernels_cpu.F90:2526-2724) for one characteristic variable.  The nonlinear weights
-// are normalised by one reciprocal of their sum (the reference divides each weight by the sum;
-// the results differ in the last bit only).
-// vp[l-1], vm[l-1] hold the reference's vp(m,l), vm(m,l), l = 1..2*WS; i = iweno = WS.
-template <class R, int WS>
-__device__ __forceinline__ R wenorec(const R (&vp)[2 * WS], const R (&vm)[2 * WS], int ord, int version,
-                                     R betascale) {
-  auto VP = [&](int l) -> R { return vp[l - 1]; };
-  auto VM = [&](int l) -> R { return vm[l - 1]; };
-  constexpr int i = WS;
-  const R eps6 = R(0.000001);
-  if (ord == 1) {
-    return VP(i) + VM(i + 1);
+// One side of wenorec_1d (kernels_cpu.F90:2526-2724): v[0 .. 2WS-2] in upwind order (the upwind
+// cell of the face at v[WS-1]) scaled so that its smoothness indicators are divided by the
+// reference's scale, eps2 = 1e-6 in that scaling.  The side's value is base + num/den.
+// The indicators and candidates are written in first and second differences d, s of the points:
+// beta_k = 13/12 s_k^2 + 1/4 b_k^2 with b_k = 3 d - d', d + d', d' - 3 d, and candidate k minus the
+// upwind cell is (3 d + 2 s)/6 or (3 d - s)/6; the weights' common factors (1/4 of the indicators,
+// 1/10 of the weights) cancel.  With the projection of weno_flux a face of the FP64 y pass executes
+// 880 FP64 instructions (central faces of its warp included) where the point values, with the fluxes
+// projected beside the states and IEEE quotients, took 1415.
+template <class R, int WS, bool WZ>
+__device__ __forceinline__ void weno_side(const R (&v)[2 * WS - 1], int ord, R eps2, R& base, R& num, R& den) {
+  constexpr int c = WS - 1;
+  base = v[c];
+  num = R(0);
+  den = R(1);
+  if (ord == 1) return;
+  if constexpr (WS >= 3) {
+    if (ord == 3) {
+      const R d0 = v[c - 1] - v[c - 2], d1 = v[c] - v[c - 1], d2 = v[c + 1] - v[c], d3 = v[c + 2] - v[c + 1];
+      const R s0 = d1 - d0, s1 = d2 - d1, s2 = d3 - d2;
+      const R b0 = R(3) * d1 - d0, b1 = d1 + d2, b2 = d3 - R(3) * d2;
+      const R k = R(13.0 / 3.0);
+      const R t3 = R(3) * d1;
+      const R r0 = R(2) * s0 + t3, r1 = R(2) * s1 + t3, r2 = R(3) * d2 - s2;  // 6 (candidate - base)
+      R n0, n1, n2;
+      if constexpr (!WZ) {
+        const R eps = R(4) * eps2;
+        const R e0 = b0 * b0 + ((k * s0) * s0 + eps), e1 = b1 * b1 + ((k * s1) * s1 + eps),
+                e2 = b2 * b2 + ((k * s2) * s2 + eps);
+        // omega_k = (d_k/e_k^2) / sum, written over the common denominator
+        const R p12 = e1 * e2, p02 = e0 * e2, p01 = e0 * e1;
+        n0 = p12 * p12;
+        n1 = R(6) * (p02 * p02);
+        n2 = R(3) * (p01 * p01);
+      } else {
+        // WENO-Z, omega_k = d_k (beta_k + tau)/(beta_k + eps); eps is a single-precision literal in
+        // the reference
+        const R eps = R(4.0 * static_cast<double>(1.e-35f) / 0.000001) * eps2;
+        const R e0 = b0 * b0 + (k * s0) * s0, e1 = b1 * b1 + (k * s1) * s1, e2 = b2 * b2 + (k * s2) * s2;
+        const R tau = fabs(e0 - e2) + eps;
+        if constexpr (sizeof(R) == sizeof(double)) {
+          const R f0 = e0 + eps, f1 = e1 + eps, f2 = e2 + eps;
+          n0 = (e0 + tau) * (f1 * f2);
+          n1 = R(6) * ((e1 + tau) * (f0 * f2));
+          n2 = R(3) * ((e2 + tau) * (f0 * f1));
+        } else {  // the products of two eps leave the FP32 range
+          n0 = R(1) / ((e0 + eps) / (e0 + tau));
+          n1 = R(6) / ((e1 + eps) / (e1 + tau));
+          n2 = R(3) / ((e2 + eps) / (e2 + tau));
+        }
+      }
+      den = n0 + n1 + n2;
+      num = (n0 * r0 + n1 * r1 + n2 * r2) * R(1.0 / 6.0);
+      return;
+    }
   }
   if constexpr (WS >= 2) {
     if (ord == 2) {
-      const R dwe0 = R(1.0) / R(3.0), dwe1 = R(2.0) / R(3.0);
-      R a = VP(i) - VP(i - 1), b = VP(i + 1) - VP(i);
-      R bp0 = betascale * (a * a), bp1 = betascale * (b * b);
-      R c = VM(i + 2) - VM(i + 1), d = VM(i + 1) - VM(i);
-      R bm0 = betascale * (c * c), bm1 = betascale * (d * d);
-      R tp0 = eps6 + bp0, tp1 = eps6 + bp1, tm0 = eps6 + bm0, tm1 = eps6 + bm1;
-      bp0 = dwe0 / (tp0 * tp0);
-      bm0 = dwe0 / (tm0 * tm0);
-      bp1 = dwe1 / (tp1 * tp1);
-      bm1 = dwe1 / (tm1 * tm1);
-      R rsp, rsm;
-      recip_pair((R(0) + bp0) + bp1, (R(0) + bm0) + bm1, rsp, rsm);
-      bp0 = bp0 * rsp; bp1 = bp1 * rsp; bm0 = bm0 * rsm; bm1 = bm1 * rsm;
-      R vminus = bp0 * (-VP(i - 1) + R(3) * VP(i)) + bp1 * (VP(i) + VP(i + 1));
-      R vplus = bm0 * (-VM(i + 2) + R(3) * VM(i + 1)) + bm1 * (VM(i) + VM(i + 1));
-      return R(0.5) * (vminus + vplus);
-    }
-  }
-  if constexpr (WS >= 3) {
-    if (ord == 3) {
-      const R dwe[3] = {R(1.0) / R(10.0), R(6.0) / R(10.0), R(3.0) / R(10.0)};
-      const R d0 = R(13.0) / R(12.0), d1 = R(1.0) / R(4.0);
-      const R c0 = R(1.0) / R(3.0), c1 = R(5.0) / R(6.0), c2 = R(-1.0) / R(6.0), c3 = R(-7.0) / R(6.0),
-              c4 = R(11.0) / R(6.0);
-      R bp[3], bm[3];
-      {
-        R a = VP(i) - R(2) * VP(i + 1) + VP(i + 2), b = R(3) * VP(i) - R(4) * VP(i + 1) + VP(i + 2);
-        bp[2] = d0 * (a * a) + d1 * (b * b);
-        a = VP(i - 1) - R(2) * VP(i) + VP(i + 1);
-        b = VP(i - 1) - VP(i + 1);
-        bp[1] = d0 * (a * a) + d1 * (b * b);
-        a = VP(i) - R(2) * VP(i - 1) + VP(i - 2);
-        b = R(3) * VP(i) - R(4) * VP(i - 1) + VP(i - 2);
-        bp[0] = d0 * (a * a) + d1 * (b * b);
-        a = VM(i + 1) - R(2) * VM(i) + VM(i - 1);
-        b = R(3) * VM(i + 1) - R(4) * VM(i) + VM(i - 1);
-        bm[2] = d0 * (a * a) + d1 * (b * b);
-        a = VM(i + 2) - R(2) * VM(i + 1) + VM(i);
-        b = VM(i + 2) - VM(i);
-        bm[1] = d0 * (a * a) + d1 * (b * b);
-        a = VM(i + 1) - R(2) * VM(i + 2) + VM(i + 3);
-        b = R(3) * VM(i + 1) - R(4) * VM(i + 2) + VM(i + 3);
-        bm[0] = d0 * (a * a) + d1 * (b * b);
-      }
-#pragma unroll
-      for (int l = 2; l >= 0; --l) {
-        bp[l] = betascale * bp[l];
-        bm[l] = betascale * bm[l];
-      }
-      if (version == 0) {
-        // omega_l = (d_l / t_l) / sum_k (d_k / t_k), t_l = (eps + beta_l)^2, formed with one
-        // division per side: omega_l = d_l prod_{m != l} t_m / sum_k d_k prod_{m != k} t_m
-        // (the same weights; the products stay far inside the exponent range for eps = 1e-6)
-        R tp[3], tm[3];
-#pragma unroll
-        for (int l = 0; l < 3; ++l) {
-          const R a = eps6 + bp[l], b = eps6 + bm[l];
-          tp[l] = a * a;
-          tm[l] = b * b;
-        }
-        const R np0 = dwe[0] * (tp[1] * tp[2]), np1 = dwe[1] * (tp[0] * tp[2]), np2 = dwe[2] * (tp[0] * tp[1]);
-        const R nm0 = dwe[0] * (tm[1] * tm[2]), nm1 = dwe[1] * (tm[0] * tm[2]), nm2 = dwe[2] * (tm[0] * tm[1]);
-        R rsp, rsm;
-        recip_pair((np0 + np1) + np2, (nm0 + nm1) + nm2, rsp, rsm);
-        bp[0] = np0 * rsp; bp[1] = np1 * rsp; bp[2] = np2 * rsp;
-        bm[0] = nm0 * rsm; bm[1] = nm1 * rsm; bm[2] = nm2 * rsm;
-      } else {
-        // eps40 is a single-precision literal in the reference
-        const R eps40 = R(static_cast<double>(1.e-35f));
-        R tau5p = fabs(bp[0] - bp[2]) + eps40;
-        R tau5m = fabs(bm[0] - bm[2]) + eps40;
-#pragma unroll
-        for (int l = 0; l < 3; ++l) {
-          bp[l] = (bp[l] + eps40) / (bp[l] + tau5p);
-          bm[l] = (bm[l] + eps40) / (bm[l] + tau5m);
-        }
-        R sump = R(0), summ = R(0);
-#pragma unroll
-        for (int l = 0; l < 3; ++l) {
-          bp[l] = dwe[l] / bp[l];
-          bm[l] = dwe[l] / bm[l];
-          sump = sump + bp[l];
-          summ = summ + bm[l];
-        }
-        R rsp, rsm;
-        recip_pair(sump, summ, rsp, rsm);
-#pragma unroll
-        for (int l = 0; l < 3; ++l) {
-          bp[l] = bp[l] * rsp;
-          bm[l] = bm[l] * rsm;
-        }
-      }
-      R vminus = bp[2] * (c0 * VP(i) + c1 * VP(i + 1) + c2 * VP(i + 2)) +
-                 bp[1] * (c2 * VP(i - 1) + c1 * VP(i) + c0 * VP(i + 1)) +
-                 bp[0] * (c0 * VP(i - 2) + c3 * VP(i - 1) + c4 * VP(i));
-      R vplus = bm[2] * (c0 * VM(i + 1) + c1 * VM(i) + c2 * VM(i - 1)) +
-                bm[1] * (c2 * VM(i + 2) + c1 * VM(i + 1) + c0 * VM(i)) +
-                bm[0] * (c0 * VM(i + 3) + c3 * VM(i + 2) + c4 * VM(i + 1));
-      return vminus + vplus;
+      const R d1 = v[c] - v[c - 1], d2 = v[c + 1] - v[c];
+      const R e0 = d1 * d1 + eps2, e1 = d2 * d2 + eps2;
+      const R n0 = e1 * e1, n1 = R(2) * (e0 * e0);
+      den = n0 + n1;
+      num = R(0.5) * (n0 * d1 + n1 * d2);
+      return;
     }
   }
   if constexpr (WS >= 4) {
-    if (ord == 4) {
-      const R dwe[4] = {R(1.0) / R(35.0), R(12.0) / R(35.0), R(18.0) / R(35.0), R(4.0) / R(35.0)};
-      const R d1 = R(1.0) / R(36.0), d2 = R(13.0) / R(12.0), d3 = R(781.0) / R(720.0);
-      auto sq = [](R a) { return a * a; };
-      R bp[4], bm[4];
-      bp[3] = d1 * sq(-11 * VP(i) + 18 * VP(i + 1) - 9 * VP(i + 2) + 2 * VP(i + 3)) +
-              d2 * sq(2 * VP(i) - 5 * VP(i + 1) + 4 * VP(i + 2) - VP(i + 3)) +
-              d3 * sq(-VP(i) + 3 * VP(i + 1) - 3 * VP(i + 2) + VP(i + 3));
-      bp[2] = d1 * sq(-2 * VP(i - 1) - 3 * VP(i) + 6 * VP(i + 1) - VP(i + 2)) +
-              d2 * sq(VP(i - 1) - 2 * VP(i) + VP(i + 1)) + d3 * sq(-VP(i - 1) + 3 * VP(i) - 3 * VP(i + 1) + VP(i + 2));
-      bp[1] = d1 * sq(VP(i - 2) - 6 * VP(i - 1) + 3 * VP(i) + 2 * VP(i + 1)) +
-              d2 * sq(VP(i - 1) - 2 * VP(i) + VP(i + 1)) + d3 * sq(-VP(i - 2) + 3 * VP(i - 1) - 3 * VP(i) + VP(i + 1));
-      bp[0] = d1 * sq(-2 * VP(i - 3) + 9 * VP(i - 2) - 18 * VP(i - 1) + 11 * VP(i)) +
-              d2 * sq(-VP(i - 3) + 4 * VP(i - 2) - 5 * VP(i - 1) + 2 * VP(i)) +
-              d3 * sq(-VP(i - 3) + 3 * VP(i - 2) - 3 * VP(i - 1) + VP(i));
-      bm[3] = d1 * sq(-11 * VM(i + 1) + 18 * VM(i) - 9 * VM(i - 1) + 2 * VM(i - 2)) +
-              d2 * sq(2 * VM(i + 1) - 5 * VM(i) + 4 * VM(i - 1) - VM(i - 2)) +
-              d3 * sq(-VM(i + 1) + 3 * VM(i) - 3 * VM(i - 1) + VM(i - 2));
-      bm[2] = d1 * sq(-2 * VM(i + 2) - 3 * VM(i + 1) + 6 * VM(i) - VM(i - 1)) +
-              d2 * sq(VM(i + 2) - 2 * VM(i + 1) + VM(i)) + d3 * sq(-VM(i + 2) + 3 * VM(i + 1) - 3 * VM(i) + VM(i - 1));
-      bm[1] = d1 * sq(VM(i + 3) - 6 * VM(i + 2) + 3 * VM(i + 1) + 2 * VM(i)) +
-              d2 * sq(VM(i + 2) - 2 * VM(i + 1) + VM(i)) + d3 * sq(-VM(i + 3) + 3 * VM(i + 2) - 3 * VM(i + 1) + VM(i));
-      bm[0] = d1 * sq(-2 * VM(i + 4) + 9 * VM(i + 3) - 18 * VM(i + 2) + 11 * VM(i + 1)) +
-              d2 * sq(-VM(i + 4) + 4 * VM(i + 3) - 5 * VM(i + 2) + 2 * VM(i + 1)) +
-              d3 * sq(-VM(i + 4) + 3 * VM(i + 3) - 3 * VM(i + 2) + VM(i + 1));
-      R sump = R(0), summ = R(0);
+    const R k1 = R(1.0 / 36.0), k2 = R(13.0 / 12.0), k3 = R(781.0 / 720.0);
+    auto sq = [](R a) { return a * a; };
+    const R a0 = v[c - 3], a1 = v[c - 2], a2 = v[c - 1], a3 = v[c], a4 = v[c + 1], a5 = v[c + 2], a6 = v[c + 3];
+    R b[4];
+    b[3] = k1 * sq(-11 * a3 + 18 * a4 - 9 * a5 + 2 * a6) + k2 * sq(2 * a3 - 5 * a4 + 4 * a5 - a6) +
+           k3 * sq(-a3 + 3 * a4 - 3 * a5 + a6);
+    b[2] = k1 * sq(-2 * a2 - 3 * a3 + 6 * a4 - a5) + k2 * sq(a2 - 2 * a3 + a4) + k3 * sq(-a2 + 3 * a3 - 3 * a4 + a5);
+    b[1] = k1 * sq(a1 - 6 * a2 + 3 * a3 + 2 * a4) + k2 * sq(a2 - 2 * a3 + a4) + k3 * sq(-a1 + 3 * a2 - 3 * a3 + a4);
+    b[0] = k1 * sq(-2 * a0 + 9 * a1 - 18 * a2 + 11 * a3) + k2 * sq(-a0 + 4 * a1 - 5 * a2 + 2 * a3) +
+           k3 * sq(-a0 + 3 * a1 - 3 * a2 + a3);
+    const R dw[4] = {R(1), R(12), R(18), R(4)};
+    // with the indicators relative to eps in FP32, whose range is too narrow for the weights' squares
+    const R sc = sizeof(R) == sizeof(double) ? R(1) : R(1) / eps2;
 #pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        bp[l] = betascale * bp[l];
-        bm[l] = betascale * bm[l];
-      }
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        R tp = eps6 + bp[l], tm = eps6 + bm[l];
-        bp[l] = dwe[l] / (tp * tp);
-        bm[l] = dwe[l] / (tm * tm);
-        sump = sump + bp[l];
-        summ = summ + bm[l];
-      }
-      R rsp, rsm;
-      recip_pair(sump, summ, rsp, rsm);
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        bp[l] = bp[l] * rsp;
-        bm[l] = bm[l] * rsm;
-      }
-      R vminus = bp[3] * (6 * VP(i) + 26 * VP(i + 1) - 10 * VP(i + 2) + 2 * VP(i + 3)) +
-                 bp[2] * (-2 * VP(i - 1) + 14 * VP(i) + 14 * VP(i + 1) - 2 * VP(i + 2)) +
-                 bp[1] * (2 * VP(i - 2) - 10 * VP(i - 1) + 26 * VP(i) + 6 * VP(i + 1)) +
-                 bp[0] * (-6 * VP(i - 3) + 26 * VP(i - 2) - 46 * VP(i - 1) + 50 * VP(i));
-      R vplus = bm[3] * (6 * VM(i + 1) + 26 * VM(i) - 10 * VM(i - 1) + 2 * VM(i - 2)) +
-                bm[2] * (-2 * VM(i + 2) + 14 * VM(i + 1) + 14 * VM(i) - 2 * VM(i - 1)) +
-                bm[1] * (2 * VM(i + 3) - 10 * VM(i + 2) + 26 * VM(i + 1) + 6 * VM(i)) +
-                bm[0] * (-6 * VM(i + 4) + 26 * VM(i + 3) - 46 * VM(i + 2) + 50 * VM(i + 1));
-      return (vminus + vplus) / R(24);
+    for (int l = 0; l < 4; ++l) {
+      const R e = sc * (b[l] + eps2);
+      b[l] = dw[l] / (e * e);
     }
+    den = b[0] + b[1] + b[2] + b[3];
+    base = R(0);
+    num = (b[3] * (6 * a3 + 26 * a4 - 10 * a5 + 2 * a6) + b[2] * (-2 * a2 + 14 * a3 + 14 * a4 - 2 * a5) +
+           b[1] * (2 * a1 - 10 * a2 + 26 * a3 + 6 * a4) + b[0] * (-6 * a0 + 26 * a1 - 46 * a2 + 50 * a3)) *
+          R(1.0 / 24.0);
   }
-  return R(0);
+}
+// wenorec_1d of one variable: the two sides of the face, p in upwind order from the left, m from the
+// right.  FP64 takes one reciprocal for both (the denominators are positive and stay far inside the
+// exponent range); the FP32 range is too narrow for their product.
+template <class R, int WS, bool WZ>
+__device__ __forceinline__ R weno_rec(const R (&p)[2 * WS - 1], const R (&m)[2 * WS - 1], int ord, R eps2) {
+  R bp, np, dp, bm, nm, dm;
+  weno_side<R, WS, WZ>(p, ord, eps2, bp, np, dp);
+  weno_side<R, WS, WZ>(m, ord, eps2, bm, nm, dm);
+  if constexpr (sizeof(R) == sizeof(double)) return (bp + bm) + (np * dm + nm * dp) * rcp_pos(dp * dm);
+  else return (bp + bm) + (fdiv(np, dp) + fdiv(nm, dm));
 }
 
 // Central energy-preserving split-form flux (kernels_cpu.F90:462-612 for x; same in y, z).
-// DIR: 0 x, 1 y, 2 z.  Points of st are at offsets -(S-1)..S (index o + S - 1).  KG = false
-// instantiates the default nkeep = 0 form at compile time (the general KEEP(n) branch, with its
-// divisions, otherwise shapes the register allocation of the whole flux kernel).
-template <class R, int DIR, int LB, int S, bool KG = true>
-__device__ __forceinline__ void central_flux(const Geom& g, const Stencil<R, S>& st, int lmax, int nkeep_in,
-                                             bool zero_flux, R (&fh)[5], R (&fl)[5]) {
+// DIR: 0 x, 1 y, 2 z.  The general form: KEEP(n) (nkeep != 0), and the default nkeep = 0 in FP32.
+// The sums over the stencil are formed in R, those over their orders l and the flux in FP64: face
+// fluxes leave in FP64, so that the differences of neighbouring faces do not lose the mixed form's
+// digits to the FP32 rounding of their final sums.
+template <class R, int DIR, int LB, int S, bool KG, class LN>
+__device__ __forceinline__ void central_flux_general(const Geom& g, const LN& ln, int lmax, int nkeep_in,
+                                                     bool zero_flux, double (&f)[5]) {
   const int nkeep = KG ? nkeep_in : 0;
   const R rgas0 = R(g.rgas0);
+  Stencil<R, S> st;
   R pp[2 * S], ee[2 * S];
 #pragma unroll
-  for (int q = 0; q < 2 * S; ++q) {
+  for (int q = S - LB; q < S + LB; ++q) {
+    st.rho[q] = ln(0, q); st.u[q] = ln(1, q); st.v[q] = ln(2, q); st.w[q] = ln(3, q);
+    st.h[q] = ln(4, q); st.t[q] = ln(5, q);
     pp[q] = st.t[q] * st.rho[q] * rgas0;
     // e = H - p/rho - |u|^2/2 with p/rho = R T taken directly (the reference divides p by rho;
     // the two differ in the last bit only and the division is the costliest operation here)
     ee[q] = st.h[q] - st.t[q] * rgas0 - R(0.5) * (st.u[q] * st.u[q] + st.v[q] * st.v[q] + st.w[q] * st.w[q]);
   }
-  R ft1 = 0, ft2 = 0, ft3 = 0, ft4 = 0, ft5 = 0, ft6 = 0;
-  R lt1 = 0, lt2 = 0, lt3 = 0, lt4 = 0, lt5 = 0, lt6 = 0;  // compensation (mixed form)
+  double ft[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
   for (int l = 1; l <= LB; ++l) {
     if (l <= lmax) {
@@ -373,68 +303,135 @@ __device__ __forceinline__ void central_flux(const Geom& g, const Stencil<R, S>&
           }
         }
       }
-      const R cl = R(g.coeff[lmax - 1][l - 1]);
-      acc_prod(ft1, lt1, cl, uvs1);
-      acc_prod(ft2, lt2, cl, uvs2);
-      acc_prod(ft3, lt3, cl, uvs3);
-      acc_prod(ft4, lt4, cl, uvs4);
-      acc_prod(ft5, lt5, cl, (nkeep >= 0 ? (uvs5_i + uvs5_k + uvs5_p) : uvs5));
-      acc_prod(ft6, lt6, cl, uvs6);
+      const double cl = g.coeff[lmax - 1][l - 1];
+      ft[0] = ft[0] + cl * double(uvs1);
+      ft[1] = ft[1] + cl * double(uvs2);
+      ft[2] = ft[2] + cl * double(uvs3);
+      ft[3] = ft[3] + cl * double(uvs4);
+      ft[4] = ft[4] + cl * double(nkeep >= 0 ? (uvs5_i + uvs5_k + uvs5_p) : uvs5);
+      ft[5] = ft[5] + cl * double(uvs6);
     }
   }
-  // scaling by 1/4 and 1/2 is exact, so the compensation terms scale with their sums
-  fh[0] = R(0.25) * ft1; fl[0] = R(0.25) * lt1;
-  fh[1] = R(0.25) * ft2; fl[1] = R(0.25) * lt2;
-  fh[2] = R(0.25) * ft3; fl[2] = R(0.25) * lt3;
-  fh[3] = R(0.25) * ft4; fl[3] = R(0.25) * lt4;
-  fh[4] = R(0.25) * ft5; fl[4] = R(0.25) * lt5;
-  if (zero_flux) {
 #pragma unroll
-    for (int m = 0; m < 5; ++m) fh[m] = fl[m] = R(0);
-  }
-  acc_add(fh[1 + DIR], fl[1 + DIR], R(0.5) * ft6);
-  fl[1 + DIR] = fl[1 + DIR] + R(0.5) * lt6;
+  for (int m = 0; m < 5; ++m) f[m] = zero_flux ? 0.0 : 0.25 * ft[m];
+  f[1 + DIR] = f[1 + DIR] + 0.5 * ft[5];
 }
+
+// nkeep = 0 in FP64, pair by pair: the sum over the orders l and the pairs (a, b) of an order is
+// one over all pairs with the coefficient of l = b - a on each, taken lower point by lower point,
+// so that LB + 1 points are held instead of 2 LB (the registers of a flux kernel are set by this
+// branch and the characteristic one: see XF_MINB_D).
+template <int DIR, int LB, int S, class LN>
+__device__ __forceinline__ void central_flux_pairs(const Geom& g, const LN& ln, int lmax, bool zero_flux,
+                                                   double (&f)[5]) {
+  const double rgas0 = g.rgas0;
+  struct Pt {
+    double rho, v[3], pp, ee;
+  };
+  auto load = [&](int q) {
+    Pt a;
+    a.rho = ln(0, q);
+    a.v[0] = ln(1, q); a.v[1] = ln(2, q); a.v[2] = ln(3, q);
+    const double rt = ln(5, q) * rgas0;
+    a.pp = rt * a.rho;
+    // e = H - p/rho - |u|^2/2 with p/rho = R T
+    a.ee = ln(4, q) - rt - 0.5 * (a.v[0] * a.v[0] + a.v[1] * a.v[1] + a.v[2] * a.v[2]);
+    return a;
+  };
+  const double* cf = g.coeff[lmax - 1];
+  double f1 = 0, fv[3] = {0, 0, 0}, fe = 0, fp = 0;
+  Pt up[LB];
+#pragma unroll
+  for (int u = 0; u < LB; ++u) up[u] = load(S + u);
+#pragma unroll
+  for (int m = 0; m < LB; ++m) {  // lower point S-1-m with the upper points S .. S+LB-1-m
+    const Pt a = load(S - 1 - m);
+#pragma unroll
+    for (int u = 0; u < LB; ++u) {
+      const int l = m + u + 1;
+      if (l <= LB && l <= lmax) {
+        const Pt& b = up[u];
+        const double cl = cf[l - 1];
+        const double uv = cl * ((a.v[DIR] + b.v[DIR]) * (a.rho + b.rho));
+        f1 = f1 + uv;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) fv[d] = fv[d] + uv * (a.v[d] + b.v[d]);
+        fe = fe + uv * ((a.ee + b.ee) + (a.v[0] * b.v[0] + a.v[1] * b.v[1] + a.v[2] * b.v[2]));
+        fe = fe + (4.0 * cl) * (a.v[DIR] * b.pp + b.v[DIR] * a.pp);
+        fp = fp + cl * (a.pp + b.pp);
+      }
+    }
+  }
+  f[0] = zero_flux ? 0.0 : 0.5 * f1;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) f[1 + d] = zero_flux ? 0.0 : 0.25 * fv[d];
+  f[4] = zero_flux ? 0.0 : 0.25 * fe;
+  f[1 + DIR] = f[1 + DIR] + fp;
+}
+
+// KG = false: nkeep = 0 fixed at compile time (the KEEP(n) divisions would otherwise shape the
+// register allocation of the whole flux kernel).
+template <class R, int DIR, int LB, int S, bool KG, class LN>
+__device__ __forceinline__ void central_flux(const Geom& g, const LN& ln, int lmax, int nkeep, bool zero_flux,
+                                             double (&f)[5]) {
+  if constexpr (sizeof(R) == sizeof(double) && !KG) central_flux_pairs<DIR, LB, S>(g, ln, lmax, zero_flux, f);
+  else central_flux_general<R, DIR, LB, S, KG>(g, ln, lmax, nkeep, zero_flux, f);
+}
+
+// A thread's own values in shared memory, for the FP64 form (st apart; a = 0: in registers).  They
+// are volatile for the same reason as the ring's.
+template <class R>
+struct Scr {
+  unsigned a, st;
+  __device__ __forceinline__ void put(int q, R v) const {
+    if constexpr (sizeof(R) == sizeof(double)) asm volatile("st.shared.f64 [%0], %1;" ::"r"(a + q * st), "d"(v));
+  }
+  __device__ __forceinline__ R get(int q) const {
+    R v = R(0);
+    if constexpr (sizeof(R) == sizeof(double)) asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a + q * st));
+    return v;
+  }
+};
 
 // Characteristic WENO flux: compute_roe_average (kernels_cpu.F90:3013-3089), eigenvectors_{x,y,z}
 // (:2728-2782, :2842-2896, :2956-3010), local Lax-Friedrichs splitting with the stencil maximum
-// of |u_n -+ c| (:614-675) and wenorec_1d; back-projection with the right eigenvectors (:677-683).
+// of |u_n -+ c| (:614-675) and wenorec_1d; back-projection with the right eigenvectors (:677-683),
+// accumulated in FP64 in both forms.
 // TP: thermally perfect gas (Newton for the Roe-averaged temperature, gamma(T) per point; FP64).
 // WZ: WENO-Z weights (weno_version = 1) instead of WENO-JS, fixed at compile time.
-template <class R, int DIR, int WS, int S, bool TP = false, bool WZ = false>
-__device__ __forceinline__ void weno_flux(const Geom& g, const Stencil<R, S>& st, int ord, R (&fh)[5],
-                                          R (&fl)[5], R* __restrict__ gs, int gstride, const R* __restrict__ cpt,
-                                          long long cstr) {
+//
+// The stencil is read point by point, again where it is needed again, and the fields are taken one
+// after another: what a thread holds between them are the projections s + a, s - a and the pressure
+// of its points.
+template <class R, int DIR, int WS, int S, bool TP, bool WZ, class LN>
+__device__ __forceinline__ void weno_flux(const Geom& g, const LN& ln, int ord, double (&f)[5], const Scr<R>& scr) {
   static_assert(!TP || sizeof(R) == sizeof(double), "the thermally perfect gas is an FP64 path");
+  constexpr int NP = 2 * WS - 1;
   const R rgas0 = R(g.rgas0);
-  const int o0 = S - 1, o1 = S;  // the two points adjacent to the face
-  // Roe average
-  R uu = st.u[o0], vv = st.v[o0], ww = st.w[o0], h = st.h[o0];
-  R r = fdiv(st.rho[o1], st.rho[o0]);
-  r = fsqrt_pos(r);
-  R rho = r * st.rho[o0];
-  R rp1 = fdiv(R(1), r + R(1));
-  uu = (r * st.u[o1] + uu) * rp1;
-  vv = (r * st.v[o1] + vv) * rp1;
-  ww = (r * st.w[o1] + ww) * rp1;
-  h = (r * st.h[o1] + h) * rp1;
-  R qq = R(0.5) * (uu * uu + vv * vv + ww * ww);
-  R hbar = h - qq - R(g.cp_last) * R(g.t0);
-  R tt, gamloc;
+  constexpr int t1 = DIR == 0 ? 1 : 0;
+  constexpr int t2 = DIR == 2 ? 1 : 2;
+  constexpr int q0 = S - WS;  // the first point used
+  // Roe average of the two points adjacent to the face
+  R vel[3], h, r, rp1;
+  {
+    const R ra = ln(0, S - 1), rb = ln(0, S);
+    if constexpr (sizeof(R) == sizeof(double)) r = rb * rsqrt_pos(ra * rb);  // sqrt(rb/ra)
+    else r = fsqrt_pos(fdiv(rb, ra));
+    rp1 = rcp_pos(r + R(1));
+#pragma unroll
+    for (int d = 0; d < 3; ++d) vel[d] = (r * ln(1 + d, S) + ln(1 + d, S - 1)) * rp1;
+    h = (r * ln(4, S) + ln(4, S - 1)) * rp1;
+  }
+  const R qq = R(0.5) * (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]);
+  const R hbar = h - qq - R(g.cp_last) * R(g.t0);
+  R c, ci, b1, b2, b3;
   if constexpr (TP) {
     // Newton on h(T) from the Roe average of the two temperatures (compute_roe_average)
-    const R t_start = (r * st.t[o1] + st.t[o0]) * rp1;
-    tt = tp_newton(g, g.cpc, hbar, t_start);
-    gamloc = gamloc_of_t(g, tt);
-  } else {
-    tt = R(g.t0) + fdiv(hbar, R(g.cp0));
-    gamloc = R(g.gamloc);
-  }
-  R cc = gamloc * tt * rgas0;
-  R c, ci, b1, b2, b3;
-  const R p_rho = tt * rgas0;
-  const R etot = h - tt * rgas0;
-  if constexpr (TP) {
+    const R t_start = (r * ln(5, S) + ln(5, S - 1)) * rp1;
+    const R tt = tp_newton(g, g.cpc, hbar, t_start);
+    const R gamloc = gamloc_of_t(g, tt);
+    const R cc = gamloc * tt * rgas0;
+    const R rho = r * ln(0, S - 1), p_rho = tt * rgas0, etot = h - tt * rgas0;
     const R gm1loc = gamloc - R(1);
     c = sqrt(cc);
     ci = R(1) / c;
@@ -446,186 +443,167 @@ __device__ __forceinline__ void weno_flux(const Geom& g, const Stencil<R, S>& st
     // constant gamma: p_e = rho (gamma - 1), so b2 = (gamma - 1)/c^2 and rho p_rho/p_e =
     // p_rho/(gamma - 1); one reciprocal square root gives c and 1/c (the reference forms three
     // quotients and a square root here: the results differ in the last bits)
-    ci = rsqrt(cc);
+    const R tt = sizeof(R) == sizeof(double) ? R(g.t0) + hbar * R(g.rcp0) : R(g.t0) + fdiv(hbar, R(g.cp0));
+    const R p_rho = tt * rgas0, cc = R(g.gamloc) * p_rho, etot = h - p_rho;
+    ci = rsqrt_pos(cc);
     c = cc * ci;
     const R ci2 = ci * ci;
     b2 = R(g.gm1) * ci2;
     b1 = p_rho * ci2 - b2 * (etot - R(2) * qq);
     b3 = etot - p_rho * R(g.rgm1);
   }
-  const R vn = DIR == 0 ? uu : (DIR == 1 ? vv : ww);
-  constexpr int t1 = DIR == 0 ? 1 : 0;
-  constexpr int t2 = DIR == 2 ? 1 : 2;
   // stencil maximum of the characteristic speeds (offsets -WS+1 .. WS)
   R ev0 = R(-1), ev1 = R(-1), ev4 = R(-1);
 #pragma unroll
   for (int l = 0; l < 2 * WS; ++l) {
-    const int q = l + S - WS;
-    const R vnq = DIR == 0 ? st.u[q] : (DIR == 1 ? st.v[q] : st.w[q]);
-#if SB_CACHE_C
-    static_assert(!TP, "the cached sound speed assumes a calorically perfect gas");
-    const R cs = st.c[q];
-#else
+    const R vnq = ln(1 + DIR, q0 + l);
     R cs;
-    if constexpr (sizeof(R) == sizeof(double)) {
-      cs = __ldg(cpt + q * cstr);  // the aux pass's sound speed of the point (FP64 form)
-    } else {
-      const R gq = TP ? R(gamloc_of_t(g, double(st.t[q]))) : R(g.gamloc);
-      cs = fsqrt_pos(gq * R(g.rgas0) * st.t[q]);
-    }
-#endif
-    ev0 = fmax(fabs(vnq - cs), ev0);
-    ev1 = fmax(fabs(vnq), ev1);
-    ev4 = fmax(fabs(vnq + cs), ev4);
+    if constexpr (sizeof(R) == sizeof(double)) cs = ln(F_C, q0 + l);  // the aux pass's sound speed (FP64 form)
+    else cs = fsqrt_pos(R(g.gamloc) * rgas0 * ln(5, q0 + l));
+    ev0 = max_of(fabs(vnq - cs), ev0);
+    ev1 = max_of(fabs(vnq), ev1);
+    ev4 = max_of(fabs(vnq + cs), ev4);
   }
-  const R betascale_a = R(g.wbs_a), betascale_b = R(g.wbs_b);
-  // Projection of the stencil's conserved states U and fluxes F onto the five characteristic
-  // fields, point by point, using the structure of the left eigenvectors (the reference forms
-  // the five dot products el(:,m).U one field at a time): with dq = Roe velocity . X(2:4),
-  // s = b1 X1 + b2 (X5 - dq) and a = ci (vn X1 - X(normal momentum)),
-  //   P1 = (s + a)/2, P2 = X1 - s, P3 = X(t1) - v_t1 X1, P4 = X(t2) - v_t2 X1, P5 = (s - a)/2.
-  // The split values g+- = (P(F) +- lambda_m P(U))/2 of every point and field go to this
-  // thread's scratch.  wenorec_1d reads g+ at the points l = 1 .. 2WS-1 and g- at l = 2 .. 2WS
-  // whatever its order (vp(i-WS+1 .. i+WS-1), vm(i-WS+2 .. i+WS) with i = WS), so each side keeps
-  // 2WS-1 values: gs[((m*(2WS-1) + l)*2 + side) * gstride], l counted from the first point used.
-  const R lam[5] = {ev0, ev1, ev1, ev1, ev4};
-  const R vel[3] = {uu, vv, ww};
-#pragma unroll
-  for (int l = 0; l < 2 * WS; ++l) {
-    const int q = l + S - WS;
-    const R rr = st.rho[q], u1 = st.u[q], v1 = st.v[q], w1 = st.w[q], h1 = st.h[q];
-    const R vq[3] = {u1, v1, w1};
-    const R rhovn = rr * vq[DIR];
-    const R pp = rr * st.t[q] * rgas0;
-    R U[5], F[5];
-    U[0] = rr; U[1] = rr * u1; U[2] = rr * v1; U[3] = rr * w1; U[4] = rr * h1 - pp;
-    F[0] = rhovn; F[1] = u1 * rhovn; F[2] = v1 * rhovn; F[3] = w1 * rhovn; F[4] = h1 * rhovn;
-    F[1 + DIR] = F[1 + DIR] + pp;
-    R PU[5], PF[5];
-#pragma unroll
-    for (int side = 0; side < 2; ++side) {
-      const R* X = side == 0 ? U : F;
-      R* P = side == 0 ? PU : PF;
-      const R dq = uu * X[1] + vv * X[2] + ww * X[3];
-      const R sv = b1 * X[0] + b2 * (X[4] - dq);
-      const R av = ci * (vn * X[0] - X[1 + DIR]);
-      P[0] = R(0.5) * (sv + av);
-      P[1] = X[0] - sv;
-      P[2] = X[1 + t1] - vel[t1] * X[0];
-      P[3] = X[1 + t2] - vel[t2] * X[0];
-      P[4] = R(0.5) * (sv - av);
-    }
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      const R cm = R(0.5) * (PF[m] + lam[m] * PU[m]);
-      if (l < 2 * WS - 1) gs[((m * (2 * WS - 1) + l) * 2) * gstride] = cm;
-      if (l > 0) gs[((m * (2 * WS - 1) + l - 1) * 2 + 1) * gstride] = PF[m] - cm;
-    }
-  }
-  // reconstruction, one characteristic field per iteration (rolled: one copy of wenorec)
+  // Projection from the structure of the left eigenvectors and of the flux: with
+  // U = rho (1, u, v, w, E) and F = u_n U + p (0, n, u_n), P(F) = u_n P(U) + p P(0, n, u_n), so that
+  // only U is projected.  s = rho (b1 + b2 (E - u_Roe.u)), a = rho ci (vn - u_n) give
+  //   P1 = (s + a)/2, P2 = rho - s, P3 = rho (u_t1 - v_t1), P4 = rho (u_t2 - v_t2), P5 = (s - a)/2
+  // and the split values are (u_n +- lambda_m) P_m(U) + p P_m(0, n, u_n), kept as 4 (m = 1, 5) and 2
+  // times the reference's g+-, exactly, undone after weno_rec.  wenorec_1d reads g+ at the points
+  // 1 .. 2WS-1 and g- at 2 .. 2WS whatever its order; the g- side is kept in upwind order from the
+  // right.  sg scales FP32 densities (a power of two near 1/(rho0 u0)).
+  constexpr bool D = sizeof(R) == sizeof(double);
+  const R sg = D ? R(1) : R(g.wsg_a), isg = D ? R(1) : R(g.wsg_ai);
+  auto rho_at = [&](int q) { return D ? ln(0, q) : ln(0, q) * sg; };
   R fi[5];
-  SB_UNROLL_(SB_WENO_UNROLL)
-  for (int m = 0; m < 5; ++m) {
-    R gp[2 * WS], gm[2 * WS];
+  // the two shear fields
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    const int t = m == 0 ? t1 : t2;
+    R gp[NP], gm[NP];
 #pragma unroll
     for (int l = 0; l < 2 * WS; ++l) {
-      gp[l] = l < 2 * WS - 1 ? gs[((m * (2 * WS - 1) + l) * 2) * gstride] : R(0);
-      gm[l] = l > 0 ? gs[((m * (2 * WS - 1) + l - 1) * 2 + 1) * gstride] : R(0);
+      const R un = ln(1 + DIR, q0 + l);
+      const R pt = rho_at(q0 + l) * (ln(1 + t, q0 + l) - vel[t]);
+      if (l < 2 * WS - 1) gp[l] = (un + ev1) * pt;
+      if (l > 0) gm[2 * WS - 1 - l] = (un - ev1) * pt;
     }
-    const R bs = (m == 2 || m == 3) ? betascale_b : betascale_a;
-    const R f = wenorec<R, WS>(gp, gm, ord, WZ ? 1 : 0, bs);
+    fi[2 + m] = weno_rec<R, WS, WZ>(gp, gm, ord, R(D ? g.weps_b : g.wepsf_ab) * R(4)) * (R(0.5) * isg);
+  }
+  // the acoustic and the entropy fields
+  R A[2 * WS], B[2 * WS], pr[2 * WS];
 #pragma unroll
-    for (int mm = 0; mm < 5; ++mm)
-      if (mm == m) fi[mm] = f;
+  for (int l = 0; l < 2 * WS; ++l) {
+    const int q = q0 + l;
+    const R rr = rho_at(q), rt = ln(5, q) * rgas0;
+    const R vq[3] = {ln(1, q), ln(2, q), ln(3, q)};
+    const R de = (ln(4, q) - rt) - (vel[0] * vq[0] + vel[1] * vq[1] + vel[2] * vq[2]);
+    const R sv = rr * (b2 * de + b1);
+    const R av = ci * (rr * (vel[DIR] - vq[DIR]));
+    if constexpr (D) {
+      scr.put(2 * l, sv + av);
+      scr.put(2 * l + 1, sv - av);
+    } else {
+      A[l] = sv + av;
+      B[l] = sv - av;
+    }
+    pr[l] = rr * rt;
+  }
+  const R epsa = R(D ? g.weps_a : g.wepsf_a);
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    R gp[NP], gm[NP];
+#pragma unroll
+    for (int l = 0; l < 2 * WS; ++l) {
+      const R un = ln(1 + DIR, q0 + l);
+      R al, bl, prl;
+      if constexpr (D) {
+        al = m != 1 ? scr.get(2 * l) : R(0);
+        bl = m != 0 ? scr.get(2 * l + 1) : R(0);
+      } else {
+        al = A[l];
+        bl = B[l];
+      }
+      prl = pr[l];
+      const R ps = (prl * b2) * (vel[DIR] - un);
+      const R pc = prl * ci;
+      const R P = m == 0 ? al : (m == 1 ? bl : rho_at(q0 + l) - R(0.5) * (al + bl));
+      const R Q = m == 0 ? -(ps + pc) : (m == 1 ? pc - ps : ps);
+      const R lam = m == 0 ? ev0 : (m == 1 ? ev4 : ev1);
+      if (l < 2 * WS - 1) gp[l] = (un + lam) * P + Q;
+      if (l > 0) gm[2 * WS - 1 - l] = (un - lam) * P + Q;
+    }
+    const R v = weno_rec<R, WS, WZ>(gp, gm, ord, epsa * (m == 2 ? R(4) : R(16))) * ((m == 2 ? R(0.5) : R(0.25)) * isg);
+    fi[m == 0 ? 0 : (m == 1 ? 4 : 1)] = v;
   }
   // back-projection with the right eigenvectors, er(m,:) = (1, u - c n, h - vn c) for m = 1,
-  // (1, u, b3) for m = 2, (0, e_t, v_t) for m = 3, 4, (1, u + c n, h + vn c) for m = 5,
-  // accumulated term by term (compensated in the mixed form)
+  // (1, u, b3) for m = 2, (0, e_t, v_t) for m = 3, 4, (1, u + c n, h + vn c) for m = 5
+  const double F0 = fi[0], F1 = fi[1], F2 = fi[2], F3 = fi[3], F4 = fi[4];
+  const double vd[3] = {double(vel[0]), double(vel[1]), double(vel[2])};
+  const double fa = F0 + F4, fd = double(c) * (F4 - F0);
+  f[0] = fa + F1;
 #pragma unroll
-  for (int m = 0; m < 5; ++m) fh[m] = fl[m] = R(0);
-  acc_add(fh[0], fl[0], fi[0]);
-  acc_add(fh[0], fl[0], fi[1]);
-  acc_add(fh[0], fl[0], fi[4]);
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    acc_prod(fh[1 + d], fl[1 + d], vel[d], fi[0]);
-    acc_prod(fh[1 + d], fl[1 + d], vel[d], fi[1]);
-    acc_prod(fh[1 + d], fl[1 + d], vel[d], fi[4]);
-    if (d == DIR) {
-      acc_prod(fh[1 + d], fl[1 + d], -c, fi[0]);
-      acc_prod(fh[1 + d], fl[1 + d], c, fi[4]);
-    }
-    if (d == t1) acc_add(fh[1 + d], fl[1 + d], fi[2]);
-    if (d == t2) acc_add(fh[1 + d], fl[1 + d], fi[3]);
-  }
-  acc_prod(fh[4], fl[4], h - vn * c, fi[0]);
-  acc_prod(fh[4], fl[4], b3, fi[1]);
-  acc_prod(fh[4], fl[4], vel[t1], fi[2]);
-  acc_prod(fh[4], fl[4], vel[t2], fi[3]);
-  acc_prod(fh[4], fl[4], h + vn * c, fi[4]);
+  for (int d = 0; d < 3; ++d) f[1 + d] = vd[d] * f[0] + (d == DIR ? fd : (d == t1 ? F2 : F3));
+  f[4] = double(h) * fa + vd[DIR] * fd + double(b3) * F1 + vd[t1] * F2 + vd[t2] * F3;
 }
 
 // Rusanov (component-wise local Lax-Friedrichs) WENO flux of the *_hybrid_rusanov kernels
 // (kernels_cpu.F90:692-941 for x, same in y and z): stencil maximum of |u_n -+ c|, split
 // values of the conserved fluxes, wenorec with the scales of wenorec_1d_rusanov (:2325-2523).
-template <class R, int DIR, int WS, int S, bool TP = false, bool WZ = false>
-__device__ __forceinline__ void rusanov_flux(const Geom& g, const Stencil<R, S>& st, int ord, R (&fh)[5], R (&fl)[5],
-                                             const R* __restrict__ cpt, long long cstr) {
+template <class R, int DIR, int WS, int S, bool TP, bool WZ, class LN>
+__device__ __forceinline__ void rusanov_flux(const Geom& g, const LN& ln, int ord, double (&f)[5]) {
   static_assert(!TP || sizeof(R) == sizeof(double), "the thermally perfect gas is an FP64 path");
+  constexpr int NP = 2 * WS - 1;
+  constexpr int q0 = S - WS;
   const R rgas0 = R(g.rgas0);
   R evmax = R(-1);
 #pragma unroll
   for (int l = 0; l < 2 * WS; ++l) {
-    const int q = l + S - WS;
-    const R un = DIR == 0 ? st.u[q] : (DIR == 1 ? st.v[q] : st.w[q]);
+    const R un = ln(1 + DIR, q0 + l);
     R c;
-    if constexpr (sizeof(R) == sizeof(double)) {
-      c = __ldg(cpt + q * cstr);
-    } else {
-      const R gq = TP ? R(gamloc_of_t(g, double(st.t[q]))) : R(g.gamloc);
-      c = fsqrt_pos(gq * rgas0 * st.t[q]);
-    }
-    const R evm = fmax(fabs(un - c), fabs(un + c));
-    evmax = fmax(evm, evmax);
+    if constexpr (sizeof(R) == sizeof(double)) c = ln(F_C, q0 + l);
+    else c = fsqrt_pos(R(g.gamloc) * rgas0 * ln(5, q0 + l));
+    evmax = max_of(max_of(fabs(un - c), fabs(un + c)), evmax);
   }
-  R bsc[5];
-  bsc[0] = R(g.wbs_a);
-  bsc[1] = R(g.wbs_b);
-  bsc[2] = bsc[1];
-  bsc[3] = bsc[1];
-  bsc[4] = R(g.wbs_c);
 #pragma unroll 1
   for (int m = 0; m < 5; ++m) {
-    R gp[2 * WS], gm[2 * WS];
+    // FP32 values are scaled by a power of two near the square root of the indicators' scale
+    R sg = R(1), isg = R(1), eps;
+    if constexpr (sizeof(R) == sizeof(double)) {
+      eps = m == 0 ? g.weps_a : (m == 4 ? g.weps_c : g.weps_b);
+    } else {
+      sg = m == 0 ? R(g.wsg_a) : (m == 4 ? R(g.wsg_c) : R(g.wsg_b));
+      isg = m == 0 ? R(g.wsg_ai) : (m == 4 ? R(g.wsg_ci) : R(g.wsg_bi));
+      eps = m == 0 ? R(g.wepsf_a) : (m == 4 ? R(g.wepsf_c) : R(g.wepsf_b));
+    }
+    R gp[NP], gm[NP];
 #pragma unroll
     for (int l = 0; l < 2 * WS; ++l) {
-      const int q = l + S - WS;
-      const R rho = st.rho[q], h = st.h[q];
-      const R vel[3] = {st.u[q], st.v[q], st.w[q]};
-      const R rhou = rho * vel[DIR];
-      const R pp = rho * st.t[q] * rgas0;
-      const R rhoevm = rho * evmax;
+      const int q = q0 + l;
+      const R rho = ln(0, q);
+      const R un = ln(1 + DIR, q);
+      const R rhou = rho * un;
       R evm, c;
       if (m == 0) {
         evm = rhou;
-        c = R(0.5) * (evm + rhoevm);
+        c = R(0.5) * (evm + rho * evmax);
       } else if (m == 4) {
+        const R h = ln(4, q);
         evm = h * rhou;
-        c = R(0.5) * (evm + evmax * (rho * h - pp));
+        c = R(0.5) * (evm + evmax * (rho * h - rho * ln(5, q) * rgas0));
       } else {
-        const R vd = m == 1 ? vel[0] : (m == 2 ? vel[1] : vel[2]);
+        const R vd = ln(m, q);
         evm = vd * rhou;
-        if (m == 1 + DIR) evm = evm + pp;
-        c = R(0.5) * (evm + rhoevm * vd);
+        if (m == 1 + DIR) evm = evm + rho * ln(5, q) * rgas0;
+        c = R(0.5) * (evm + rho * evmax * vd);
       }
-      gp[l] = c;
-      gm[l] = evm - c;
+      if (l < 2 * WS - 1) gp[l] = sg * c;
+      if (l > 0) gm[2 * WS - 1 - l] = sg * (evm - c);
     }
-    const R bs = m == 0 ? bsc[0] : (m == 4 ? bsc[4] : bsc[1]);
-    const R f = wenorec<R, WS>(gp, gm, ord, WZ ? 1 : 0, bs);
+    const R v = weno_rec<R, WS, WZ>(gp, gm, ord, eps) * isg;
 #pragma unroll
     for (int mm = 0; mm < 5; ++mm)
-      if (mm == m) { fh[mm] = f; fl[mm] = R(0); }
+      if (mm == m) f[mm] = double(v);
   }
 }
 

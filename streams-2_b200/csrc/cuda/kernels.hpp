@@ -135,8 +135,9 @@ struct BoxRec {
   Scalars* sc;
   double cfl;
   int sly, nsy, slz, nsz;  // march segments (length, count) of the y and z passes
-  unsigned xg[3];          // grid of the x pass (one-dimensional)
-  unsigned nb_vol, nb_pt, nb_y, nb_z;  // blocks of the aux pass, pointwise passes, y and z passes
+  int nwy, nwz;            // and the warps of their blocks
+  int xgrp, pad;           // x pass: groups of 32 faces a warp takes
+  unsigned nb_x, nb_vol, nb_pt, nb_y, nb_z;  // blocks of the aux pass, pointwise passes, y and z passes
   unsigned nb_vs;                      // blocks of the staged viscous pass
   unsigned nb_up;                      // blocks of the update and time-step passes
 };
@@ -145,12 +146,20 @@ struct BlockRef {
   unsigned box, local;
 };
 enum BatchKind { BK_VOL = 0, BK_PT, BK_X, BK_Y, BK_Z, BK_VS, BK_UP, BK_NUM };
+// blocks of a y or z pass of one size: warps, longest segment, place in the block table
+struct MarchLaunch {
+  int nwarps, maxseg;
+  long long off;
+  unsigned cnt;
+};
 struct BoxTable {
   int nbox = 0;
   BoxRec* rec = nullptr;       // device
   BlockRef* blocks = nullptr;  // device: the blocks of each kind, box after box
   long long off[BK_NUM] = {};
   unsigned cnt[BK_NUM] = {};
+  int xslots = 0;  // x pass: points of a warp's buffer (the box with the shortest rows)
+  std::vector<MarchLaunch> march[2];  // the launches of the y and z passes
   Geom g0{};  // host copy of the first box's geometry: the group's common configuration
 };
 // Group key of a geometry (boxes with equal keys share launches), -1 for a box whose stage

@@ -35,38 +35,32 @@ namespace {
 
 constexpr int AUX_NT = 256;
 constexpr int XF_TX = 32, XF_TY = 4, XF_NT = XF_TX * XF_TY;  // x faces: 4 row-warps per block
-constexpr int MT_NT = 128;                                     // march kernels
-// Resident blocks per SM asked of the register allocator for the FP64 and FP32 instantiations
-// of the flux kernels (measured on the 1024x256x192 boundary layer; the kernels are FP64-latency
-// bound, so resident warps pay).  FP64 x pass: 4 blocks of 128 threads (128 registers, no
-// spills; 16.5 against 18.6 ms per step at 3 blocks), which the WENO scratch of 2WS-1 values a
-// side allows (51 KB a block).  FP64 march passes: 3 blocks (the y pass without a register
-// window: at 4 blocks its reloads miss L1, 18.8 against 17.3 ms; the windowed passes spill
-// 176-228 bytes at 4 blocks).  FP32, with the Newton-refined quotients: 6 blocks for the x pass
-// (12.31 against 12.89 ms per step at 5, the same at 7) and 5 for the march passes (y 12.11,
-// z 14.72 against 12.36, 15.33 at 4; z 17.1 at 6).
+// y / z passes: blocks of LW = 4 warps, up to MT_MAXW in small boxes; segments of at most MT_SEG cells
+constexpr int MT_MAXW = 9, MT_SEG = 2048;
+// Registers of the flux kernels, as the threads an SM shall hold (y / z: 65536 / MT_MAXT_* registers
+// for blocks of any size) or the blocks of 128 (x, WENO faces).  The FP64 kernels want 128 registers
+// (1024x256x192 boundary layer, ms per step: y 12.2, z 13.6, x 11.5 at 16 warps per SM; at 20 warps
+// and 96 registers they spill 80-180 bytes: 13.2, 15.1, 12.1), the FP32 ones 80 (1024x256x128 shock
+// interaction: z 7.4, y 5.6 at 24 warps against 7.2, 5.7 at 20; 512x256x256 channel: z 5.9, y 3.1
+// against 6.1, 3.4; x 3.3 at 24 against 3.8 at 20).  The WENO face kernels' scattered stencils are
+// held in registers: 3 blocks (6.5 against 7.2 ms at 4) and 4 (1.9 against 2.1 ms at 5) in FP32.
+#ifndef MT_MAXT_D
+#define MT_MAXT_D 512
+#endif
+#ifndef MT_MAXT_F
+#define MT_MAXT_F 768
+#endif
 #ifndef XF_MINB_D
 #define XF_MINB_D 4
 #endif
 #ifndef XF_MINB_F
 #define XF_MINB_F 6
 #endif
-#ifndef MT_MINB_D
-#define MT_MINB_D 3
+#ifndef WF_MINB_D
+#define WF_MINB_D 3
 #endif
-// y / z passes: the stencil window slides along the line in registers (1), or every face loads
-// its stencil afresh (0: no window held across the WENO branch, fewer registers).  Measured on
-// the boundary layer: y 17.3 (reload) against 18.2 ms per step (window), z 21.9 (reload)
-// against 21.3 (window): the z planes are a plane apart, so the reloads leave L1.
-#ifndef SB_MARCH_WINDOW_Y
-#define SB_MARCH_WINDOW_Y 0
-#endif
-#ifndef SB_MARCH_WINDOW_Z
-#define SB_MARCH_WINDOW_Z 1
-#endif
-// the viscous pass with its operands staged in shared memory (1) or read per use (0)
-#ifndef SB_VISC_TILED
-#define SB_VISC_TILED 1
+#ifndef WF_MINB_F
+#define WF_MINB_F 4
 #endif
 // shared-memory carve-out (percent) preferred by the WENO face kernels: their listed faces'
 // stencil loads are scattered and live on L1 hits (developed boundary layer 1024x256x192: 5.0
@@ -74,12 +68,9 @@ constexpr int MT_NT = 128;                                     // march kernels
 #ifndef SB_WF_CARVEOUT
 #define SB_WF_CARVEOUT 72
 #endif
-#ifndef MT_MINB_F
-#define MT_MINB_F 5
-#endif
-// the channel's FP32 z pass (force_rhs partials) keeps 4: at 5 it spills 244 bytes
-#ifndef MT_MINB_F_CH
-#define MT_MINB_F_CH 4
+// the viscous pass with its operands staged in shared memory (1) or read per use (0)
+#ifndef SB_VISC_TILED
+#define SB_VISC_TILED 1
 #endif
 // the viscous pass: the staged FP64 pass at 3 blocks of 256 threads per SM (80 registers; 7.42
 // against 7.57 ms per step at 4 blocks and 64 registers on the 1024x256x192 boundary layer), the
@@ -399,24 +390,22 @@ __device__ __forceinline__ R sensor_at(const Geom& g, const R* __restrict__ s, i
   return s[iidx(g, i, j, k)];
 }
 // bcextr_var (kernels_cpu.F90:6199-6254) then bcswap_var: periodic wrap, otherwise nearest interior
-template <class R>
-__device__ __forceinline__ R div3_at(const Geom& g, const R* __restrict__ d, int i, int j, int k) {
+__device__ __forceinline__ long long div3_idx(const Geom& g, int i, int j, int k) {
   if (i < 1 || i > g.nx) i = g.periodic[0] ? wrap(i, g.nx) : (i < 1 ? 1 : g.nx);
   if (j < 1 || j > g.ny) j = g.periodic[1] ? wrap(j, g.ny) : (j < 1 ? 1 : g.ny);
   if (k < 1 || k > g.nz) k = g.periodic[2] ? wrap(k, g.nz) : (k < 1 ? 1 : g.nz);
-  return d[iidx(g, i, j, k)];
+  return iidx(g, i, j, k);
+}
+template <class R>
+__device__ __forceinline__ R div3_at(const Geom& g, const R* __restrict__ d, int i, int j, int k) {
+  return d[div3_idx(g, i, j, k)];
 }
 
-// Per-thread scratch of the WENO characteristic projections (dynamic shared memory of the flux
-// kernels, 5 fields x (2WS-1) points x 2 sides per thread, thread-interleaved)
+// 1/(x(i+1)-x(i-1)) of a line of direction d in R
 template <class R>
-__device__ __forceinline__ R* weno_scratch() {
-  extern __shared__ __align__(16) unsigned char sb_dyn_smem[];
-  return reinterpret_cast<R*>(sb_dyn_smem);
-}
-template <class R, int WS>
-constexpr size_t weno_scratch_bytes(int nthreads) {
-  return (size_t)nthreads * 5 * (2 * WS - 1) * 2 * sizeof(R);
+__device__ __forceinline__ R line_r(const Geom& g, int d, int i) {
+  if constexpr (sizeof(R) == sizeof(double)) return __ldg(g.vrl[d] + i);
+  else return __ldg(g.vrlf[d] + i);
 }
 
 template <int DIR>
@@ -479,8 +468,7 @@ __host__ __device__ __forceinline__ long long wface_count(const Geom& g) {
                   : (DIR == 1 ? (long long)g.nx * (g.ny + 1) * g.nz : (long long)g.nx * g.ny * (g.nz + 1));
 }
 
-// Flux at a face from a loaded stencil window (points p-(S-1) .. p+S of face p):
-// hi + lo is the face flux (lo = 0 in the FP64 form).  FS holds the flux variant flags of a
+// Flux at a face in FP64 from its stencil in memory.  FS holds the flux variant flags of a
 // kernel instantiation: bit 0 the component-wise (Rusanov) WENO splitting, bit 1 the thermally
 // perfect gas, bit 2 a central flux with nkeep != 0 (otherwise nkeep = 0 at compile time), bit 3
 // the WENO-Z weights (otherwise WENO-JS).  Options fixed per kernel instantiation keep the code
@@ -488,128 +476,213 @@ __host__ __device__ __forceinline__ long long wface_count(const Geom& g) {
 // (measured: nkeep 10-18 %, the WENO version 3-10 % of the flux passes).
 // The WENO flux of face p (characteristic or component-wise splitting), order reduced near
 // non-periodic boundaries as ep_ord_change says.
-template <class R, int DIR, int LB, int WS, int S, int FS = 0>
-__device__ __forceinline__ void weno_face(const Geom& g, const Stencil<R, S>& st, int p, R (&hi)[5], R (&lo)[5],
-                                          R* __restrict__ gs, int gstride, const R* __restrict__ cpt, long long cstr) {
-  const int ep = face_ep<DIR>(g, p);
+template <class R, int DIR, int LB, int WS, int S, int FS, class LN>
+__device__ __forceinline__ void weno_face(const Geom& g, const LN& ln, int ep, double (&f)[5], const Scr<R>& scr) {
   const int ord = max(WS + ep, 1);
   if constexpr ((FS & 1) != 0)
-    rusanov_flux<R, DIR, WS, S, (FS & 2) != 0, (FS & 8) != 0>(g, st, ord, hi, lo, cpt, cstr);
+    rusanov_flux<R, DIR, WS, S, (FS & 2) != 0, (FS & 8) != 0>(g, ln, ord, f);
   else
-    weno_flux<R, DIR, WS, S, (FS & 2) != 0, (FS & 8) != 0>(g, st, ord, hi, lo, gs, gstride, cpt, cstr);
+    weno_flux<R, DIR, WS, S, (FS & 2) != 0, (FS & 8) != 0>(g, ln, ord, f, scr);
 }
 
-template <class R, int DIR, int LB, int WS, int S, int FS = 0>
-__device__ __forceinline__ void window_flux(const Geom& g, const Stencil<R, S>& st, bool ishk, int p,
-                                            R (&hi)[5], R (&lo)[5], R* __restrict__ gs, int gstride,
-                                            const R* __restrict__ cpt, long long cstr, bool split, int wa, int wb) {
+template <class R, int DIR, int LB, int WS, int S, int FS, class LN>
+__device__ __forceinline__ void face_flux(const Geom& g, const LN& ln, bool ishk, int p, int ep, double (&f)[5],
+                                          const Scr<R>& scr, bool split, int wa, int wb) {
   const int nd = DIR == 0 ? g.nx : (DIR == 1 ? g.ny : g.nz);
   if (!ishk) {
-    const int ep = face_ep<DIR>(g, p);
     const int lmax = max(g.lmax_base + ep, 1);
     const bool zf = (p == 0 && g.fzf[2 * DIR] == 1) || (p == nd && g.fzf[2 * DIR + 1] == 1);
-    central_flux<R, DIR, LB, S, (FS & 4) != 0>(g, st, lmax, g.nkeep, zf, hi, lo);
+    central_flux<R, DIR, LB, S, (FS & 4) != 0>(g, ln, lmax, g.nkeep, zf, f);
   } else if (SB_WENO_SPLIT && split) {
     // the WENO faces come from the face buffer
-    const R* fb = static_cast<const R*>(g.wface);
     const long long wf = wface_index<DIR>(g, p, wa, wb);
 #pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      hi[m] = __ldg(fb + m * g.nwface + wf);
-      lo[m] = sizeof(R) == sizeof(double) ? R(0) : __ldg(fb + (5 + m) * g.nwface + wf);
-    }
+    for (int m = 0; m < 5; ++m) f[m] = __ldg(g.wface + m * g.nwface + wf);
   } else {
-    weno_face<R, DIR, LB, WS, S, FS>(g, st, p, hi, lo, gs, gstride, cpt, cstr);
+    weno_face<R, DIR, LB, WS, S, FS>(g, ln, ep, f, scr);
   }
 }
 
-template <class R, int S>
-__device__ __forceinline__ void load_point(const Geom& g, Stencil<R, S>& st, int q, const R* __restrict__ aux,
-                                           long long n, long long a) {
-  st.rho[q] = __ldg(aux + a);
-  st.u[q] = __ldg(aux + n + a);
-  st.v[q] = __ldg(aux + 2 * n + a);
-  st.w[q] = __ldg(aux + 3 * n + a);
-  st.h[q] = __ldg(aux + 4 * n + a);
-  st.t[q] = __ldg(aux + 5 * n + a);
-#if SB_CACHE_C
-  st.c[q] = sqrt(R(g.gamloc) * R(g.rgas0) * st.t[q]);
-#endif
+// asynchronous copies of one value from global to shared memory
+__device__ __forceinline__ void copy_async(unsigned dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
-
-// Divergence of one variable between a face pair, in FP64: (hi_up - hi_lo) + (lo_up - lo_lo).
-template <class R>
-__device__ __forceinline__ double face_diff(R hup, R lup, R hlo, R llo) {
-  if constexpr (sizeof(R) == sizeof(double)) {
-    return double(hup) - double(hlo);
-  } else {
-    return (double(hup) - double(hlo)) + (double(lup) - double(llo));
-  }
+__device__ __forceinline__ void copy_async(unsigned dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// x faces: each warp owns one (j,k) row segment of 32 faces (i0-1 .. i0+30) and updates the 31
-// cells between them; the upper face of a cell comes from the neighbouring lane by a shuffle,
-// so no shared memory and no block barrier are needed.  fl is written (first contribution of the
-// stage, euler_x after init_flux).
+// x faces.  The faces of all rows form one sequence (row (k-1) ny + (j-1), faces p = 0..nx in a row;
+// fewer than 2^32 faces, checked at create), so that no lane idles at a row's end.  A warp takes
+// ngrp groups of 32 consecutive faces one after another (its first face is the last of the warp
+// before) and forms the cells below its faces, the lower face of a cell coming from the lane before
+// by a shuffle and from the group before through shared memory.  A group's points are copied to the
+// warp's own buffer while the group before is computed (no block barrier anywhere): 32 points and
+// 2S - 1 more for every row that the group touches, and the sensor beside them.  1024x256x192
+// boundary layer, ms per step: 16.7 with the stencil loaded by every face into registers, 13.7 read
+// from L1 as often as used, 11.5 from the buffer.
+// fl is written (first contribution of the stage, euler_x after init_flux).
+// values of a thread's scratch (Scr): the two acoustic projections of the stencil's points
+template <class R, int WS>
+constexpr int scr_vals() { return sizeof(R) == sizeof(double) ? 4 * WS : 0; }
+constexpr int XG_MAX = 8, X_SMEM_MAX = 64 * 1024;
+struct XShape {
+  int ngrp, slots;
+  unsigned nblk;
+};
+__host__ __device__ __forceinline__ int x_slots(int nx, int S) { return 32 + (2 * S - 1) * ((31 + nx) / (nx + 1) + 1); }
+template <class R, int WS>
+__host__ __device__ __forceinline__ size_t x_warp_bytes(int slots) {
+  return 2 * (size_t)((slots * XS * (int)sizeof(R) + 7) / 8 * 8 + slots * 8) + 5 * 8 + scr_vals<R, WS>() * 32 * 8;
+}
 template <class R, int LB, int WS, int FS = 0>
-__device__ __forceinline__ void d_xflux(const Geom& g, const R* __restrict__ aux,
-                                                 const double* __restrict__ sensor, double* __restrict__ fl, const Blk blk) {
-  constexpr int S = LB > WS ? LB : WS;
-  const int lane = threadIdx.x;
-  // The x faces of all rows form one sequence (row (k-1) ny + (j-1), faces p = 0..nx in a row;
-  // fewer than 2^32 faces, checked at create): warp w holds faces 31w .. 31w+31, and forms the
-  // cells between its lanes' faces within a row, so no lane idles at a row's end.
-  const unsigned nfr = (unsigned)g.nx + 1u;
+__device__ __forceinline__ void d_xflux(const Geom& g, const R* __restrict__ aux, const double* __restrict__ sensor,
+                                        double* __restrict__ fl, int ngrp, const Blk blk) {
+  constexpr int S = LB > WS ? LB : WS, W2 = 2 * S - 1, RF = ring_fields<R>();
+  extern __shared__ __align__(16) unsigned char sb_dyn_smem[];
+  const int lane = threadIdx.x, nfr = g.nx + 1, slots = x_slots(g.nx, S);
   const unsigned long long nface = (unsigned long long)nfr * g.ny * g.nz;
-  const unsigned long long f0 = (unsigned long long)(blk.x * XF_TY + threadIdx.y) * (XF_TX - 1);
-  if (f0 >= nface) return;  // whole warp leaves together
-  const bool in = f0 + lane < nface;
-  const unsigned fu = in ? (unsigned)(f0 + lane) : 0u;
-  const unsigned row = fu / nfr;
-  const int p = (int)(fu - row * nfr);  // this lane's face (between p and p+1)
-  const int j = (int)(row % (unsigned)g.ny) + 1, k = (int)(row / (unsigned)g.ny) + 1;
-  const bool face_ok = in && p >= g.eul_imin - 1 && p <= g.eul_imax;
-  R fh[5] = {0, 0, 0, 0, 0}, fo[5] = {0, 0, 0, 0, 0};
-  if (face_ok) {
-    bool ishk = false;
+  const unsigned long long fw0 = (unsigned long long)(blk.x * XF_TY + threadIdx.y) * (unsigned)(32 * ngrp - 1);
+  if (fw0 >= nface) return;  // whole warp leaves together
+  const unsigned nmine = (unsigned)min((unsigned long long)(32 * ngrp), nface - fw0);  // this warp's faces
+  unsigned char* wm = sb_dyn_smem + threadIdx.y * x_warp_bytes<R, WS>(slots);
+  const Scr<R> scr{(unsigned)__cvta_generic_to_shared(wm) + lane * 8, 32 * 8};
+  wm += scr_vals<R, WS>() * 32 * 8;
+  double* carry = reinterpret_cast<double*>(wm);  // the group before's last face
+  const unsigned pb = (unsigned)((slots * XS * (int)sizeof(R) + 7) / 8 * 8);  // bytes of a buffer's points
+  unsigned char* buf0 = wm + 5 * 8;
+  // a group's first face (p0 of the row j0, k0); the faces of a group in its first row
+  struct Pos {
+    int p, j, k;
+  };
+  auto forward = [&](Pos q, int n) {  // n faces on
+    q.p += n;
+    while (q.p >= nfr) {
+      q.p -= nfr;
+      if (++q.j > g.ny) {
+        q.j = 1;
+        ++q.k;
+      }
+    }
+    return q;
+  };
+  auto fetch = [&](const Pos& q0, int nf, int bi) {  // the points of the nf faces from q0 on
+    unsigned char* pts = buf0 + bi * (pb + slots * 8);
+    double* sen = reinterpret_cast<double*>(pts + pb);
+    const int n0 = nfr - q0.p;  // faces left in the first row
+    const int total = nf + W2 * ((q0.p + nf - 1) / nfr + 1);
+    for (int s = lane; s < total; s += 32) {
+      Pos q = q0;
+      int t = s;
+      if (t < n0 + W2) {
+        t += q.p;
+      } else {
+        t -= n0 + W2;
+        q = forward(Pos{0, q.j, q.k}, nfr);
+        while (t >= nfr + W2) {
+          t -= nfr + W2;
+          q = forward(q, nfr);
+        }
+      }
+      const int i = t - (S - 1);
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(pts) + s * (XS * (unsigned)sizeof(R));
+      const R* src = aux + gidx(g, i, q.j, q.k);
 #pragma unroll
-    for (int o = -WS + 1; o <= WS; ++o) ishk = ishk || sensor_at(g, sensor, p + o, j, k) > g.sensor_threshold;
-    Stencil<R, S> st;
-    const long long base = gidx(g, p, j, k);
-#pragma unroll
-    for (int q = 0; q < 2 * S; ++q) load_point<R, S>(g, st, q, aux, g.nvol, base + (q - (S - 1)));
-    // the FP64 form's aux holds the sound speed of every point (field 8): stencil point 0 onwards
-    const R* cpt = sizeof(R) == sizeof(double) ? aux + 7 * g.nvol + base - (S - 1) : nullptr;
-    window_flux<R, 0, LB, WS, S, FS>(g, st, ishk, p, fh, fo, weno_scratch<R>() + threadIdx.y * XF_TX + lane, XF_NT,
-                                     cpt, 1, weno_split<0>(g), j, k);
+      for (int f = 0; f < RF; ++f) copy_async(dst + f * (unsigned)sizeof(R), src + (f == F_C ? 7 : f) * g.nvol);
+      int is = i;
+      if (i < 1 || i > g.nx) is = g.periodic[0] ? wrap(i, g.nx) : 0;
+      if (is > 0) copy_async((unsigned)__cvta_generic_to_shared(sen + s), sensor + iidx(g, is, q.j, q.k));
+      else sen[s] = 0.0;  // no sensor beyond a boundary
+    }
+  };
+  Pos q0;
+  {
+    const unsigned fu = (unsigned)fw0, row = fu / (unsigned)nfr;
+    q0.p = (int)(fu - row * (unsigned)nfr);
+    q0.k = (int)(row / (unsigned)g.ny) + 1;
+    q0.j = (int)(row - (unsigned)(q0.k - 1) * (unsigned)g.ny) + 1;
   }
-  R hu[5], lu[5];
+  const bool split = weno_split<0>(g);
+  fetch(q0, (int)min(32u, nmine), 0);
+  copy_commit();
+  for (unsigned b = 0; b < nmine; b += 32) {
+    const int nf = (int)min(32u, nmine - b), bi = (b >> 5) & 1;
+    const Pos qn = forward(q0, 32);
+    // this lane's face (between the points p and p+1) and its first stencil point
+    const Pos q = forward(q0, lane);
+    const int s0 = lane + W2 * ((q0.p + lane) / nfr);
+    const int p = q.p;
+    const bool in = lane < nf;
+    const int ep = in ? face_ep<0>(g, p) : 0;
+    if (b + 32 < nmine) fetch(qn, (int)min(32u, nmine - b - 32), bi ^ 1);
+    copy_commit();
+    copy_wait<1>();
+    __syncwarp();
+    unsigned char* pts = buf0 + bi * (pb + slots * 8);
+    const double* sen = reinterpret_cast<const double*>(pts + pb);
+    double f[5] = {0, 0, 0, 0, 0};
+    if (in && p >= g.eul_imin - 1 && p <= g.eul_imax) {
+      bool ishk = false;
 #pragma unroll
-  for (int m = 0; m < 5; ++m) {
-    hu[m] = __shfl_down_sync(0xffffffffu, fh[m], 1);
-    if constexpr (sizeof(R) != sizeof(double)) lu[m] = __shfl_down_sync(0xffffffffu, fo[m], 1);
-    else lu[m] = R(0);
-  }
-  const int i = p + 1;  // cell between faces p and p+1 (the next lane's face, in this row)
-  if (lane < XF_TX - 1 && in && i <= g.nx) {
-    const bool upd = i >= g.eul_imin && i <= g.eul_imax;
-    const double met = g.dcsidx[i];
-    const long long ic = iidx(g, i, j, k);
+      for (int o = S - WS; o < S + WS; ++o) ishk = ishk | (sen[s0 + o] > g.sensor_threshold);
+      const RowPts<R> ln{(unsigned)__cvta_generic_to_shared(pts) + s0 * (XS * (unsigned)sizeof(R))};
+      face_flux<R, 0, LB, WS, S, FS>(g, ln, ishk, p, ep, f, scr, split, q.j, q.k);
+    }
+    // the cell i = p between the faces p-1 and p
+    const bool cell = in && p >= 1 && b + lane > 0;
+    const bool upd = cell && p >= g.eul_imin && p <= g.eul_imax;
+    const double met = upd ? g.dcsidx[p] : 0.0;
+    const long long ic = iidx(g, p, q.j, q.k);
 #pragma unroll
-    for (int m = 0; m < 5; ++m) fl[m * g.nint + ic] = upd ? face_diff<R>(hu[m], lu[m], fh[m], fo[m]) * met : 0.0;
+    for (int m = 0; m < 5; ++m) {
+      double lo = __shfl_up_sync(0xffffffffu, f[m], 1);
+      if (lane == 0 && b > 0) lo = carry[m];
+      if (cell) fl[m * g.nint + ic] = upd ? (f[m] - lo) * met : 0.0;
+    }
+    __syncwarp();  // the buffer and the carry have been read
+    if (lane == 31)
+#pragma unroll
+      for (int m = 0; m < 5; ++m) carry[m] = f[m];
+    q0 = qn;
   }
 }
 template <class R, int LB, int WS, int FS = 0>
-__global__ void __launch_bounds__(XF_NT, sizeof(R) == 8 ? XF_MINB_D : XF_MINB_F) k_xflux(Geom g, const R* __restrict__ aux,
-                                                 const double* __restrict__ sensor, double* __restrict__ fl) {
-  d_xflux<R, LB, WS, FS>(g, aux, sensor, fl, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
+__global__ void __launch_bounds__(XF_NT, sizeof(R) == 8 ? XF_MINB_D : XF_MINB_F)
+    k_xflux(Geom g, const R* __restrict__ aux, const double* __restrict__ sensor, double* __restrict__ fl, int ngrp) {
+  d_xflux<R, LB, WS, FS>(g, aux, sensor, fl, ngrp, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
 }
 
-// y or z faces by marching: each thread owns one line (fixed i and the other transverse index)
-// over a segment of cells, keeps the stencil window of the current face in registers (one new
-// point loaded per face), computes every face of the segment once and adds the divergence to fl.
+// y or z faces: a block owns a tile of 32 lines (consecutive i of the lines' plane, so that every
+// load is a coalesced row) over a segment of cells, and its warps take consecutive faces of the
+// segment, one each per round.  The points sit in a ring in shared memory, copied once per block
+// while the round before is computed, so that a face reads its stencil as often as it likes without
+// the address arithmetic and the latency of global loads; the warps' fluxes meet in shared memory,
+// where the cells between them find both faces.  A face is a chain of about a thousand FP64
+// operations, most of them dependent: what bounds the pass is how many are in flight (22 % of the
+// warp slots at 128 registers, FP64 pipe about 55 % in y and 50 % in z).
+// Against a thread marching alone along its line with the stencil in registers (168 of them, and
+// 51 KB of scratch per block), 1024x256x192 boundary layer: y 17.0 -> 12.2, z 20.5 -> 13.6 ms per
+// step; and since a segment takes a round per block of faces instead of a face at a time, a
+// 32x24x16 channel's z pass 93 -> 19 us, its y pass 66 -> 19 us.  What a cell adds to is read before
+// the barrier after the fluxes, which hides it behind the other warps' faces (read after it: y 12.6,
+// z 16.1; copied to shared memory a round ahead: 13.6, 17.3, the copies' own instructions).
 // The z pass also applies the grad(mu div/3) term of visflx_div_ord2_subroutine
 // (kernels_cpu.F90:3446-3480) and emits the force_rhs block partials (:3157-3193).
+//
+// Dynamic shared memory: the fluxes of a round ((warps + 1) x 5 x 32, slot 0 the previous round's
+// last face), the threads' scratch, the ring of points (the nw + 2S - 1 of a round and the nw of the
+// next, which are copied while the round's fluxes are formed), the sensor flags of the segment's
+// points (a word of 32 lanes each).
+constexpr int MARCH_SMEM_MAX = 220 * 1024;
+__host__ __device__ __forceinline__ int ring_slots(int nw, int S) { return 2 * nw + 2 * S - 1; }
+template <class R, int LB, int WS>
+size_t march_smem(int nwarps, int seglen) {
+  constexpr int S = LB > WS ? LB : WS;
+  return (size_t)(nwarps + 1) * 5 * 32 * 8 + (size_t)nwarps * 32 * scr_vals<R, WS>() * 8 +
+         (size_t)ring_slots(nwarps, S) * ring_fields<R>() * 32 * sizeof(R) + ((size_t)seglen + 2 * WS) * 4;
+}
 template <class R, int DIR, int LB, int WS, bool CH = false, int FS = 0, bool SPLIT = false>
 __device__ __forceinline__ void d_march(const Geom& g, const R* __restrict__ aux,
                                                  const double* __restrict__ sensor, double* __restrict__ fl,
@@ -619,150 +692,210 @@ __device__ __forceinline__ void d_march(const Geom& g, const R* __restrict__ aux
                                                  int istep, int seglen, int nseg, double* __restrict__ red, const Blk blk) {
   static_assert(DIR == 1 || DIR == 2, "march kernel handles y and z");
   constexpr int S = LB > WS ? LB : WS;
-  constexpr int NP = 2 * S;
-  __shared__ double rsh[5 * (MT_NT / 32)];
+  extern __shared__ __align__(16) unsigned char sb_dyn_smem[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  double* xch = reinterpret_cast<double*>(sb_dyn_smem);
+  constexpr int RF = ring_fields<R>();
+  const int nslot = ring_slots(nw, S);
+  double* scd = xch + (nw + 1) * 5 * 32;
+  const Scr<R> scr{(unsigned)__cvta_generic_to_shared(scd + threadIdx.x), blockDim.x * 8};
+  R* ring = reinterpret_cast<R*>(scd + scr_vals<R, WS>() * blockDim.x);
+  unsigned* flag = reinterpret_cast<unsigned*>(ring + nslot * RF * 32);
+  const unsigned ring_a = (unsigned)__cvta_generic_to_shared(ring) + lane * (unsigned)sizeof(R);
   const int n1 = g.nx;
   const int n2 = DIR == 1 ? g.nz : g.ny;
   const int nd = DIR == 1 ? g.ny : g.nz;
   const int emin = DIR == 1 ? g.eul_jmin : g.eul_kmin;
   const int emax = DIR == 1 ? g.eul_jmax : g.eul_kmax;
   const long long nlines = (long long)n1 * n2;
-  const long long t = (long long)blk.x * MT_NT + threadIdx.x;
   // both forms are launched; the one that the list length does not select leaves at once
   if (weno_split<DIR>(g) != SPLIT) return;
+  const unsigned tiles = (unsigned)((nlines + 31) / 32);
+  const unsigned sgi = blk.x / tiles;
+  const long long line = (long long)(blk.x - sgi * tiles) * 32 + lane;
+  const bool in = line < nlines;
+  const unsigned lu = in ? (unsigned)line : 0u, lb = lu / (unsigned)n1;
+  const int i = (int)(lu - lb * (unsigned)n1) + 1;
+  const int b = (int)lb + 1;  // k for y lines, j for z lines
+  const int c0 = emin + (int)sgi * seglen;
+  const int c1 = min(c0 + seglen - 1, emax);
+  const long long n = g.nvol, nI = g.nint;
+  const long long sd = DIR == 1 ? (long long)g.sx : (long long)g.sx * g.sy;
+  const long long base0 = DIR == 1 ? gidx(g, i, 0, b) : gidx(g, i, b, 0);  // address of c = 0
+  constexpr unsigned PB = RF * 32 * (unsigned)sizeof(R);  // bytes of a point of the ring
+  // points c0-S .. c1+S of the segment's stencils, point c in slot (c - c0 + S) mod nslot, which is
+  // s0 for ca; a warp copies a point at a time
+  auto fetch = [&](int ca, int cb, int s0) {
+    for (int c = ca + wid; c <= cb; c += nw)
+      if (in) {
+        int sl = s0 + (c - ca);
+        if (sl >= nslot) sl -= nslot;
+        const unsigned dst = ring_a + sl * PB;
+        const R* src = aux + base0 + (long long)c * sd;
+#pragma unroll
+        for (int q = 0; q < RF; ++q) copy_async(dst + q * 32 * (unsigned)sizeof(R), src + (q == F_C ? 7 : q) * n);
+      }
+  };
+  fetch(c0 - S, min(c0 - 2 + nw + S, c1 + S), 0);
+  copy_commit();
+  // the sensor flags of the points c0-WS .. c1+WS (word q: point c0-WS+q)
+  for (int q = wid; q < c1 - c0 + 1 + 2 * WS; q += nw) {
+    int c = c0 - WS + q;
+    bool on = in;
+    if (c < 1 || c > nd) {
+      on = on && g.periodic[DIR];
+      c = on ? wrap(c, nd) : 1;
+    }
+    if (on) on = (DIR == 1 ? sensor[iidx(g, i, c, b)] : sensor[iidx(g, i, b, c)]) > g.sensor_threshold;
+    const unsigned bal = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) flag[q] = bal;
+  }
   double part[5] = {0, 0, 0, 0, 0};
-  if (t < nlines * nseg) {
-    const int i = (int)(t % n1) + 1;
-    const int b = (int)((t / n1) % n2) + 1;  // k for y lines, j for z lines
-    const int sgi = (int)(t / nlines);
-    const int c0 = emin + sgi * seglen;
-    const int c1 = min(c0 + seglen - 1, emax);
-    const long long n = g.nvol, nI = g.nint;
-    const long long sd = DIR == 1 ? (long long)g.sx : (long long)g.sx * g.sy;
-    const long long base0 = DIR == 1 ? gidx(g, i, 0, b) : gidx(g, i, b, 0);  // address of c = 0
-    // sensor bits of the face p: points p-WS+1 .. p+WS at bits 0 .. 2WS-1
-    auto sensor_bit = [&](int c) -> unsigned {
-      if (c < 1 || c > nd) {
-        if (!g.periodic[DIR]) return 0u;
-        c = wrap(c, nd);
-      }
-      const double th = DIR == 1 ? sensor[iidx(g, i, c, b)] : sensor[iidx(g, i, b, c)];
-      return th > g.sensor_threshold ? 1u : 0u;
-    };
-    // preload the window and sensor bits of the face c0-2; the loop starts at the face c0-1
-    Stencil<R, S> st;
-    const int p = c0 - 2;
-    constexpr bool WIN = DIR == 1 ? SB_MARCH_WINDOW_Y != 0 : SB_MARCH_WINDOW_Z != 0;
-    if constexpr (WIN) {
-#pragma unroll
-      for (int q = 1; q < NP; ++q) load_point<R, S>(g, st, q, aux, n, base0 + (long long)(p - (S - 1) + q) * sd);
+  double f[5] = {0, 0, 0, 0, 0};
+  int sr = 0;  // slot of the round's first point, cr - S + 1
+  for (int cr = c0 - 1; cr <= c1; cr += nw) {
+    const int c = cr + wid;  // this warp's face (between the cells c and c+1)
+    const bool face = in && c <= c1;
+    const int ep = face ? face_ep<DIR>(g, c) : 0;
+    // the next round's points: their slots were last read before the barrier after the fluxes
+    {
+      int sn = sr + nw + 2 * S - 1;
+      if (sn >= nslot) sn -= nslot;
+      fetch(cr + nw + S, min(cr + 2 * nw - 1 + S, c1 + S), sn);
     }
-    unsigned mask = 0;
+    copy_commit();
+    copy_wait<1>();
+    __syncthreads();  // this round's points and (first round) the flags are there
+    if (wid == nw - 1)  // the previous round's last face
 #pragma unroll
-    for (int bq = 1; bq < 2 * WS; ++bq) mask |= sensor_bit(p - WS + 1 + bq) << bq;
-    R hlo[5] = {0, 0, 0, 0, 0}, llo[5] = {0, 0, 0, 0, 0};
-    // x(i+1)-x(i-1) and y(j+1)-y(j-1) of the z line (the grad(mu div/3) term)
-    R xdiff = R(1), ydiff = R(1);
-    if constexpr (DIR == 2) {
-      xdiff = R(g.x[i + 1] - g.x[i - 1]);
-      ydiff = R(g.y[b + 1] - g.y[b - 1]);
+      for (int m = 0; m < 5; ++m) xch[m * 32 + lane] = f[m];
+    Ring<R, 2 * S> ln;
+    {
+      int sl = sr + wid;
+      if (sl >= nslot) sl -= nslot;
+#pragma unroll
+      for (int q = 0; q < 2 * S; ++q) ln.o[q] = ring_a + (sl + q >= nslot ? sl + q - nslot : sl + q) * PB;
     }
-    for (int c = c0 - 1; c <= c1; ++c) {
-      if constexpr (WIN) {
-        // slide the window to the face c
+    sr += nw;
+    if (sr >= nslot) sr -= nslot;
+    if (face) {
+      unsigned any = 0;  // points c-WS+1 .. c+WS
 #pragma unroll
-        for (int q = 0; q < NP - 1; ++q) {
-          st.rho[q] = st.rho[q + 1]; st.u[q] = st.u[q + 1]; st.v[q] = st.v[q + 1];
-          st.w[q] = st.w[q + 1]; st.h[q] = st.h[q + 1]; st.t[q] = st.t[q + 1];
-#if SB_CACHE_C
-          st.c[q] = st.c[q + 1];
-#endif
+      for (int q = 0; q < 2 * WS; ++q) any |= flag[c + 1 - c0 + q];
+      face_flux<R, DIR, LB, WS, S, FS>(g, ln, (any >> lane) & 1u, c, ep, f, scr, SPLIT, i, b);
+    }
+    double* own = xch + (wid + 1) * 5 * 32 + lane;
+#pragma unroll
+    for (int m = 0; m < 5; ++m) own[m * 32] = f[m];
+    // what the cell c between the faces c-1 and c adds to, read before the barrier
+    const bool cell = face && c >= c0;
+    const long long ic = DIR == 1 ? iidx(g, i, c, b) : iidx(g, i, b, c);
+    double r[5] = {0, 0, 0, 0, 0}, met = 0;
+    R uu = 0, vv = 0, ww = 0, tt0 = 0, rh0 = 0, mu = 0, dv[6] = {0, 0, 0, 0, 0, 0};
+    if (cell) {
+#pragma unroll
+      for (int m = 0; m < 5; ++m) r[m] = fl[m * nI + ic];
+      met = DIR == 1 ? g.detady[c] : g.dzitdz[c];
+      if constexpr (DIR == 2) {
+        mu = __ldg(aux + 6 * n + base0 + (long long)c * sd);
+        if (g.conservative_viscous) {
+          dv[0] = __ldg(div3 + div3_idx(g, i + 1, b, c));
+          dv[1] = __ldg(div3 + div3_idx(g, i - 1, b, c));
+          dv[2] = __ldg(div3 + div3_idx(g, i, b + 1, c));
+          dv[3] = __ldg(div3 + div3_idx(g, i, b - 1, c));
+          dv[4] = __ldg(div3 + div3_idx(g, i, b, c + 1));
+          dv[5] = __ldg(div3 + div3_idx(g, i, b, c - 1));
         }
-        load_point<R, S>(g, st, NP - 1, aux, n, base0 + (long long)(c + S) * sd);
-      } else {
-        // the face's stencil, loaded afresh: the lanes of a warp hold consecutive i, so every
-        // load is one coalesced row, and the points shared with the previous face come from L1
-#pragma unroll
-        for (int q = 0; q < NP; ++q) load_point<R, S>(g, st, q, aux, n, base0 + (long long)(c - (S - 1) + q) * sd);
+        uu = ln(1, S - 1); vv = ln(2, S - 1); ww = ln(3, S - 1);  // the face's lower point
+        if constexpr (CH && sizeof(R) == sizeof(double)) {
+          rh0 = ln(0, S - 1);
+          tt0 = ln(5, S - 1);
+        }
       }
-      mask = (mask >> 1) | (sensor_bit(c + WS) << (2 * WS - 1));
-      R hhi[5], lhi[5];
-      const R* cpt = sizeof(R) == sizeof(double) ? aux + 7 * n + base0 + (long long)(c - (S - 1)) * sd : nullptr;
-      window_flux<R, DIR, LB, WS, S, FS>(g, st, mask != 0u, c, hhi, lhi, weno_scratch<R>() + threadIdx.x, MT_NT, cpt,
-                                         sd, SPLIT, i, b);
-      if (c >= c0) {
-        // cell c lies between the faces c-1 (lo) and c (hi)
-        const long long ic = DIR == 1 ? iidx(g, i, c, b) : iidx(g, i, b, c);
-        const double met = DIR == 1 ? g.detady[c] : g.dzitdz[c];
-        double f[5];
+    }
+    __syncthreads();
+    if (cell) {
+      // the lower face: the warp before, or the previous round's last
 #pragma unroll
-        for (int m = 0; m < 5; ++m) f[m] = fl[m * nI + ic] + face_diff<R>(hhi[m], lhi[m], hlo[m], llo[m]) * met;
-        if (DIR == 2) {
-          const int j = b, k = c;
-          const long long a = gidx(g, i, j, k);
-          // the cell's velocities are the stencil's point S-1 (the face c's lower point)
-          const R uu = st.u[S - 1], vv = st.v[S - 1], ww = st.w[S - 1], mu = aux[6 * n + a];
-          R sigx, sigy, sigz;
-          if (g.conservative_viscous) {
-            const R dxl = mu / xdiff;
-            const R dyl = mu / ydiff;
-            const R dzl = mu / R(g.z[k + 1] - g.z[k - 1]);
-            sigx = dxl * (div3_at(g, div3, i + 1, j, k) - div3_at(g, div3, i - 1, j, k));
-            sigy = dyl * (div3_at(g, div3, i, j + 1, k) - div3_at(g, div3, i, j - 1, k));
-            sigz = dzl * (div3_at(g, div3, i, j, k + 1) - div3_at(g, div3, i, j, k - 1));
+      for (int m = 0; m < 5; ++m) r[m] = r[m] + (f[m] - own[m * 32 - 5 * 32]) * met;
+      if (DIR == 2) {
+        const int j = b, k = c;
+        R sigx, sigy, sigz;
+        if (g.conservative_viscous) {
+          // mu times the per-line 1/(x(i+1)-x(i-1))
+          const R dxl = mu * line_r<R>(g, 0, i), dyl = mu * line_r<R>(g, 1, j), dzl = mu * line_r<R>(g, 2, k);
+          sigx = dxl * (dv[0] - dv[1]);
+          sigy = dyl * (dv[2] - dv[3]);
+          sigz = dzl * (dv[4] - dv[5]);
+        } else {
+          // visflx_div_subroutine (kernels_cpu.F90:3484-3532): order visc_order
+          const int lv = g.lmax_base;
+          R dx3 = R(0), dy3 = R(0), dz3 = R(0);
+          for (int l = 1; l <= lv; ++l) {
+            const R ccl = R(g.coeff[lv - 1][l - 1]);
+            dx3 = dx3 + ccl * (div3_at(g, div3, i + l, j, k) - div3_at(g, div3, i - l, j, k));
+            dy3 = dy3 + ccl * (div3_at(g, div3, i, j + l, k) - div3_at(g, div3, i, j - l, k));
+            dz3 = dz3 + ccl * (div3_at(g, div3, i, j, k + l) - div3_at(g, div3, i, j, k - l));
+          }
+          sigx = mu * (dx3 * R(g.dcsidx[i]));
+          sigy = mu * (dy3 * R(g.detady[j]));
+          sigz = mu * (dz3 * R(g.dzitdz[k]));
+        }
+        const R sigq = sigx * uu + sigy * vv + sigz * ww;
+        r[1] = r[1] - double(sigx);
+        r[2] = r[2] - double(sigy);
+        r[3] = r[3] - double(sigz);
+        r[4] = r[4] - double(sigq);
+        if constexpr (CH) {
+          const double dt = sc->dt;
+          const double rhodt = rhork * dt, gamdt = gamrk * dt;
+          const double fln1 = (istep > 1 ? -(rhodt * fl_prev[ic]) : 0.0) - gamdt * r[0];
+          const double fln2 = (istep > 1 ? -(rhodt * fl_prev[nI + ic]) : 0.0) - gamdt * r[1];
+          const double dy = g.yn[j + 1] - g.yn[j];
+          // density, momentum and temperature of the stage's state: the ring's in FP64, else from w
+          double rho, rhou, tt;
+          if constexpr (sizeof(R) == sizeof(double)) {
+            rho = rh0;
+            rhou = rho * uu;
+            tt = tt0;
           } else {
-            // visflx_div_subroutine (kernels_cpu.F90:3484-3532): order visc_order
-            const int lv = g.lmax_base;
-            R dx3 = R(0), dy3 = R(0), dz3 = R(0);
-            for (int l = 1; l <= lv; ++l) {
-              const R ccl = R(g.coeff[lv - 1][l - 1]);
-              dx3 = dx3 + ccl * (div3_at(g, div3, i + l, j, k) - div3_at(g, div3, i - l, j, k));
-              dy3 = dy3 + ccl * (div3_at(g, div3, i, j + l, k) - div3_at(g, div3, i, j - l, k));
-              dz3 = dz3 + ccl * (div3_at(g, div3, i, j, k + l) - div3_at(g, div3, i, j, k - l));
-            }
-            sigx = mu * (dx3 * R(g.dcsidx[i]));
-            sigy = mu * (dy3 * R(g.detady[j]));
-            sigz = mu * (dz3 * R(g.dzitdz[k]));
+            const long long a = base0 + (long long)c * sd;
+            const Prim pr = prim_from_w<false>(g, w, a, g.t0);
+            rho = pr.rho;
+            rhou = w[n + a];
+            tt = pr.tt;
           }
-          const R sigq = sigx * uu + sigy * vv + sigz * ww;
-          f[1] = f[1] - double(sigx);
-          f[2] = f[2] - double(sigy);
-          f[3] = f[3] - double(sigz);
-          f[4] = f[4] - double(sigq);
-          if constexpr (CH) {
-            const double dt = sc->dt;
-            const double rhodt = rhork * dt, gamdt = gamrk * dt;
-            double fln1 = (istep > 1 ? -(rhodt * fl_prev[ic]) : 0.0) - gamdt * f[0];
-            double fln2 = (istep > 1 ? -(rhodt * fl_prev[nI + ic]) : 0.0) - gamdt * f[1];
-            double dy = g.yn[j + 1] - g.yn[j];
-            const Prim pr = prim_from_w<(FS & 2) != 0>(g, w, a, (FS & 2) != 0 ? double(aux[5 * n + a]) : g.t0);
-            double rhou = w[n + a];
-            part[0] += fln1 * dy;
-            part[1] += fln2 * dy;
-            part[2] += pr.rho * dy;
-            part[3] += rhou * dy;
-            part[4] += rhou * dy * pr.tt;
-          }
+          part[0] += fln1 * dy;
+          part[1] += fln2 * dy;
+          part[2] += rho * dy;
+          part[3] += rhou * dy;
+          part[4] += rhou * dy * tt;
         }
-#pragma unroll
-        for (int m = 0; m < 5; ++m) fl[m * nI + ic] = f[m];
       }
 #pragma unroll
-      for (int m = 0; m < 5; ++m) {
-        hlo[m] = hhi[m];
-        llo[m] = lhi[m];
-      }
+      for (int m = 0; m < 5; ++m) fl[m * nI + ic] = r[m];
     }
   }
   if constexpr (DIR == 2 && CH) {
-    block_reduce_sum<5, MT_NT>(part, rsh);
-    if (threadIdx.x == 0)
+    // lanes, then the block's warps in order (the flux exchange is done with: reuse it)
 #pragma unroll
-      for (int r = 0; r < 5; ++r) red[(long long)blk.x * 5 + r] = part[r];
+    for (int r = 0; r < 5; ++r)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) part[r] += __shfl_down_sync(0xffffffffu, part[r], o);
+    __syncthreads();
+    if (lane == 0)
+#pragma unroll
+      for (int r = 0; r < 5; ++r) xch[r * 32 + wid] = part[r];
+    __syncthreads();
+    if (threadIdx.x < 5) {
+      double a = 0.0;
+      for (int q = 0; q < nw; ++q) a += xch[threadIdx.x * 32 + q];
+      red[(long long)blk.x * 5 + threadIdx.x] = a;
+    }
   }
 }
 template <class R, int DIR, int LB, int WS, bool CH = false, int FS = 0, bool SPLIT = false>
-__global__ void __launch_bounds__(MT_NT, sizeof(R) == 8 ? MT_MINB_D : (CH ? MT_MINB_F_CH : MT_MINB_F)) k_march(Geom g, const R* __restrict__ aux,
+__global__ void __launch_bounds__(sizeof(R) == 8 ? MT_MAXT_D : MT_MAXT_F, 1) k_march(Geom g, const R* __restrict__ aux,
                                                  const double* __restrict__ sensor, double* __restrict__ fl,
                                                  const R* __restrict__ div3,
                                                  const double* __restrict__ w, const double* __restrict__ fl_prev,
@@ -1642,58 +1775,93 @@ __global__ void __launch_bounds__(WL_NT) k_weno_list(Geom g) {
 // list; each thread loads its face's stencil as the hybrid pass would hold it).
 constexpr int WF_NT = 128;
 template <class R, int DIR, int LB, int WS, int FS>
-__global__ void __launch_bounds__(WF_NT) k_weno_faces(Geom g, const R* __restrict__ aux) {
+__global__ void __launch_bounds__(WF_NT, sizeof(R) == 8 ? WF_MINB_D : WF_MINB_F) k_weno_faces(Geom g, const R* __restrict__ aux) {
   constexpr int S = LB > WS ? LB : WS;
   const unsigned cnt = g.wcount[DIR];
   if (cnt > g.wthr[DIR]) return;  // the hybrid pass computes the WENO faces itself
   const long long n = g.nvol;
   const long long sd = DIR == 0 ? 1 : (DIR == 1 ? (long long)g.sx : (long long)g.sx * g.sy);
-  R* fb = static_cast<R*>(g.wface);
   for (unsigned e = blockIdx.x * WF_NT + threadIdx.x; e < cnt; e += gridDim.x * WF_NT) {
     const unsigned f = g.wlist[DIR][e];
     int p, a, b;
     wface_decode<DIR>(g, f, p, a, b);
     const long long base = DIR == 0 ? gidx(g, p, a, b) : (DIR == 1 ? gidx(g, a, p, b) : gidx(g, a, b, p));
-    Stencil<R, S> st;
-#pragma unroll
-    for (int q = 0; q < 2 * S; ++q) load_point<R, S>(g, st, q, aux, n, base + (q - (S - 1)) * sd);
-    const R* cpt = sizeof(R) == sizeof(double) ? aux + 7 * n + base - (S - 1) * sd : nullptr;
-    R hi[5], lo[5];
-    weno_face<R, DIR, LB, WS, S, FS>(g, st, p, hi, lo, weno_scratch<R>() + threadIdx.x, WF_NT, cpt, sd);
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      fb[m * g.nwface + f] = hi[m];
-      if constexpr (sizeof(R) != sizeof(double)) fb[(5 + m) * g.nwface + f] = lo[m];
+    const Line<R> ln{aux + base - (S - 1) * sd, n, sd};
+    double fw[5];
+    Scr<R> scr{0, 0};
+    if constexpr (scr_vals<R, WS>() > 0) {
+      __shared__ double wsc[scr_vals<R, WS>() * WF_NT];
+      scr = Scr<R>{(unsigned)__cvta_generic_to_shared(wsc + threadIdx.x), WF_NT * 8};
     }
+    weno_face<R, DIR, LB, WS, S, FS>(g, ln, face_ep<DIR>(g, p), fw, scr);
+#pragma unroll
+    for (int m = 0; m < 5; ++m) g.wface[m * g.nwface + f] = fw[m];
   }
 }
 
 inline unsigned nblocks(long long n, int nt) { return (unsigned)((n + nt - 1) / nt); }
-// blocks of the x pass: warps of 31 new faces each over the (nx+1) ny nz faces, XF_TY per block
-inline unsigned x_blocks(const Geom& g) {
+// Launch shape of the x pass: XF_TY warps a block, each of ngrp groups of 32 faces with one face
+// shared between neighbouring warps; as many groups as leave four waves of resident warps (a group
+// more saves a face in 32 and hides the copy of its points, a wave less leaves SMs idle at the end)
+inline XShape x_shape(const Geom& g) {
+  const int S = std::max(g.lmax_base, g.weno_scheme);
   const long long nface = (long long)(g.nx + 1) * g.ny * g.nz;
-  return nblocks((nface + XF_TX - 2) / (XF_TX - 1), XF_TY);
+  XShape x;
+  x.ngrp = (int)std::min<long long>(XG_MAX, std::max<long long>(1, nface / (32LL * 148 * 16 * 4)));
+  x.slots = x_slots(g.nx, S);
+  const long long per = 32LL * x.ngrp - 1;
+  x.nblk = nblocks((std::max<long long>(1, nface - 1) + per - 1) / per, XF_TY);
+  return x;
 }
 
-// Segments of a march pass: enough threads to fill the device, segments of at least 16 cells
-// (one redundant face per segment).
-inline void march_split_with(const Geom& g, int dir, long long target, int minseg, int* seglen, int* nseg,
-                             long long* nthreads) {
+// Launch shape of a y or z pass: segments of seglen cells (nseg of them on each line) and the warps
+// of a block.  The segments are at least minseg cells and at most as many as bring the pass to
+// about target threads; among the counts allowed, the one with the least estimated time is taken:
+// rounds of a segment's seglen + 1 faces over the block's warps times the blocks an SM works
+// through, of which up to MT_FREE run beside one another at no cost (a face is a long dependent
+// chain).  Blocks have LW warps; when they are fewer than the SMs can hold, up to MT_MAXW of them
+// (a function of the box alone, so that a box has the same partition in every form it runs in).
+constexpr int LW = 4, MT_FREE = 4;
+struct MarchShape {
+  int seglen, nseg, nwarps;
+  unsigned nblk;
+};
+inline MarchShape march_shape_with(const Geom& g, int dir, long long target, int minseg) {
   const int emin = dir == 1 ? g.eul_jmin : g.eul_kmin, emax = dir == 1 ? g.eul_jmax : g.eul_kmax;
   const int ncell = emax - emin + 1;
+  if (ncell < 1) return MarchShape{1, 0, LW, 0};
   const long long lines = (long long)g.nx * (dir == 1 ? g.nz : g.ny);
-  long long ns = (target + lines - 1) / lines;
-  int sl = (int)((ncell + ns - 1) / ns);
-  if (sl < minseg) sl = minseg;
-  if (sl > ncell) sl = ncell;
-  if (sl < 1) sl = 1;
-  *seglen = sl;
-  *nseg = ncell > 0 ? (ncell + sl - 1) / sl : 0;
-  *nthreads = lines * *nseg;
+  const long long tiles = (lines + 31) / 32;
+  const long long most = std::min<long long>(std::max(1, ncell / minseg), (target + lines * LW - 1) / (lines * LW));
+  // a segment's flags sit in shared memory: at most MT_SEG cells
+  const long long least = (ncell + MT_SEG - 1) / MT_SEG;
+  double best = 0.0;
+  int bn = 1;
+  for (long long ns = least; ns <= std::max(least, most); ++ns) {
+    const int sl = (int)((ncell + ns - 1) / ns);
+    const double rounds = (sl + 1 + LW - 1) / LW;
+    const double perSM = (double)((tiles * ns + 147) / 148);
+    const double cost = rounds * std::max(1.0, perSM / MT_FREE);
+    if (ns == least || cost < best) {
+      best = cost;
+      bn = (int)ns;
+    }
+  }
+  MarchShape m;
+  m.seglen = (ncell + bn - 1) / bn;
+  m.nseg = (ncell + m.seglen - 1) / m.seglen;
+  const long long blocks = tiles * m.nseg;
+  m.nblk = (unsigned)blocks;
+  const int room = (int)std::min<long long>(MT_MAXW, 148LL * MT_MAXW / std::max<long long>(1, blocks));
+  m.nwarps = LW;
+  if (room > LW) {
+    const int rounds = (m.seglen + 1 + room - 1) / room;
+    m.nwarps = std::max(LW, (m.seglen + 1 + rounds - 1) / rounds);
+  }
+  return m;
 }
-
-inline void march_split(const Geom& g, int dir, int* seglen, int* nseg, long long* nthreads) {
-  march_split_with(g, dir, g.march_threads, g.march_minseg, seglen, nseg, nthreads);
+inline MarchShape march_shape(const Geom& g, int dir) {
+  return march_shape_with(g, dir, g.march_threads, g.march_minseg);
 }
 
 // typed views of the precision-dependent buffers

@@ -52,11 +52,9 @@ void Prof::reset() {
 
 long long reduction_slots(const Geom& g) {
   long long a = (long long)nblocks(g.nint, 256) * (NRED_UPD > 9 ? NRED_UPD : 9);
-  int sl, ns;
-  long long nt;
   // the largest segment count any tuning can reach: segments of MARCH_MINSEG_MIN cells
-  march_split_with(g, 2, 1LL << 40, MARCH_MINSEG_MIN, &sl, &ns, &nt);
-  long long b = (long long)nblocks(nt, MT_NT) * 5;
+  const long long nseg = std::max(1, (g.eul_kmax - g.eul_kmin + 1 + MARCH_MINSEG_MIN - 1) / MARCH_MINSEG_MIN);
+  long long b = (((long long)g.nx * g.ny + 31) / 32) * nseg * 5;
   return a > b ? a : b;
 }
 
@@ -151,12 +149,9 @@ template <class R, int LB, int WS, int FS = 0>
 static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, double* fl_prev, double* fl_new,
                               cudaStream_t s, long long* nl) {
   const dim3 xb(XF_TX, XF_TY);
-  const unsigned xg = x_blocks(g);
-  int sly, nsy, slz, nsz;
-  long long nty, ntz;
-  march_split(g, 1, &sly, &nsy, &nty);
-  march_split(g, 2, &slz, &nsz, &ntz);
-  const unsigned gyb = nblocks(nty, MT_NT), gzb = nblocks(ntz, MT_NT);
+  const XShape xs = x_shape(g);
+  const size_t xsm = XF_TY * x_warp_bytes<R, WS>(xs.slots);
+  const MarchShape my = march_shape(g, 1), mz = march_shape(g, 2);
   R* aux = aux_of<R>(d);
   double* sensor = d.sensor;
   double* sensor_next = d.sensor_next;
@@ -165,23 +160,20 @@ static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, do
   // the mixed form's stage-3 sensor is taken in FP64 from velocities that this aux pass stores
   double* vel = (!fp64 && a.istep == 3) ? d.vel64 : nullptr;
   if (a.run_aux) aux_launch<R>(g, d, a.apply_shift, 0, K_AUX, s, nl, vel);
-  // the hybrid passes hold the WENO scratch for the steps at which they compute WENO faces
-  const size_t xsm = weno_scratch_bytes<R, WS>(XF_NT);
-  const size_t msm = weno_scratch_bytes<R, WS>(MT_NT);
-  const size_t wsm = weno_scratch_bytes<R, WS>(WF_NT);
+  const size_t ysm = march_smem<R, LB, WS>(my.nwarps, my.seglen);
+  const size_t zsm = march_smem<R, LB, WS>(mz.nwarps, mz.seglen);
   // per instantiation and device: allow more than 48 KB of dynamic shared memory
   static unsigned long long smem_set = 0;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !(smem_set & (1ULL << dev))) {
-    cudaFuncSetAttribute(k_xflux<R, LB, WS, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xsm);
-    cudaFuncSetAttribute(k_march<R, 1, LB, WS, false, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm);
-    cudaFuncSetAttribute(k_march<R, 2, LB, WS, false, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm);
-    cudaFuncSetAttribute(k_march<R, 2, LB, WS, true, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm);
+    cudaFuncSetAttribute(k_xflux<R, LB, WS, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, X_SMEM_MAX);
+    // block sizes and segments vary with the box: the most any takes
+    for (auto fn : {(const void*)k_march<R, 1, LB, WS, false, FS>, (const void*)k_march<R, 2, LB, WS, false, FS>,
+                    (const void*)k_march<R, 2, LB, WS, true, FS>, (const void*)k_march<R, 1, LB, WS, false, FS, true>,
+                    (const void*)k_march<R, 2, LB, WS, false, FS, true>, (const void*)k_march<R, 2, LB, WS, true, FS, true>})
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, MARCH_SMEM_MAX);
     if (SB_WENO_SPLIT) {
-      cudaFuncSetAttribute(k_weno_faces<R, 0, LB, WS, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
-      cudaFuncSetAttribute(k_weno_faces<R, 1, LB, WS, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
-      cudaFuncSetAttribute(k_weno_faces<R, 2, LB, WS, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
       // a larger L1 rather than a fourth block (SB_WF_CARVEOUT)
       for (auto fn : {(const void*)k_weno_faces<R, 0, LB, WS, FS>, (const void*)k_weno_faces<R, 1, LB, WS, FS>,
                       (const void*)k_weno_faces<R, 2, LB, WS, FS>})
@@ -216,10 +208,10 @@ static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, do
     *nl += 7;
   }
   if (split_on) {
-    SB_LAUNCH(d, K_WENO_FACES, s, k_weno_faces<R, 0, LB, WS, FS><<<wgrid, WF_NT, wsm, s>>>(g, aux));
+    SB_LAUNCH(d, K_WENO_FACES, s, k_weno_faces<R, 0, LB, WS, FS><<<wgrid, WF_NT, 0, s>>>(g, aux));
     ++*nl;
   }
-  SB_LAUNCH(d, K_EULER_X, s, k_xflux<R, LB, WS, FS><<<xg, xb, xsm, s>>>(g, aux, sensor, fl_new));
+  SB_LAUNCH(d, K_EULER_X, s, k_xflux<R, LB, WS, FS><<<xs.nblk, xb, xsm, s>>>(g, aux, sensor, fl_new, xs.ngrp));
   if (g.conservative_viscous && SB_VISC_TILED)
     SB_LAUNCH(d, K_VISC, s,
               k_visc_tiled<R, (FS & 2) != 0><<<visc_tiled_blocks(g), VT_NT, 0, s>>>(
@@ -244,48 +236,48 @@ static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, do
     ++*nl;
   }
   if (split_on) {
-    SB_LAUNCH(d, K_WENO_FACES, s, k_weno_faces<R, 1, LB, WS, FS><<<wgrid, WF_NT, wsm, s>>>(g, aux));
+    SB_LAUNCH(d, K_WENO_FACES, s, k_weno_faces<R, 1, LB, WS, FS><<<wgrid, WF_NT, 0, s>>>(g, aux));
     ++*nl;
   }
-  if (gyb > 0) {
+  if (my.nblk > 0) {
     SB_LAUNCH(d, K_EULER_Y, s,
-              k_march<R, 1, LB, WS, false, FS><<<gyb, MT_NT, msm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev, d.sc,
-                                                          a.rhork, a.gamrk, a.istep, sly, nsy, d.red));
+              k_march<R, 1, LB, WS, false, FS><<<my.nblk, 32 * my.nwarps, ysm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev, d.sc,
+                                                          a.rhork, a.gamrk, a.istep, my.seglen, my.nseg, d.red));
     if (split_on) {
       SB_LAUNCH(d, K_EULER_Y, s,
-                k_march<R, 1, LB, WS, false, FS, true><<<gyb, MT_NT, 0, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
-                                                                   d.sc, a.rhork, a.gamrk, a.istep, sly, nsy, d.red));
+                k_march<R, 1, LB, WS, false, FS, true><<<my.nblk, 32 * my.nwarps, ysm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
+                                                                   d.sc, a.rhork, a.gamrk, a.istep, my.seglen, my.nseg, d.red));
       ++*nl;
     }
   }
   if (split_on) {
-    SB_LAUNCH(d, K_WENO_FACES, s, k_weno_faces<R, 2, LB, WS, FS><<<wgrid, WF_NT, wsm, s>>>(g, aux));
+    SB_LAUNCH(d, K_WENO_FACES, s, k_weno_faces<R, 2, LB, WS, FS><<<wgrid, WF_NT, 0, s>>>(g, aux));
     ++*nl;
   }
   // the channel's force_rhs partials are a separate instantiation (fewer registers without them)
   if (g.channel_case) {
     SB_LAUNCH(d, K_EULER_Z, s,
-              k_march<R, 2, LB, WS, true, FS><<<gzb, MT_NT, msm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev, d.sc,
-                                                                  a.rhork, a.gamrk, a.istep, slz, nsz, d.red));
+              k_march<R, 2, LB, WS, true, FS><<<mz.nblk, 32 * mz.nwarps, zsm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev, d.sc,
+                                                                  a.rhork, a.gamrk, a.istep, mz.seglen, mz.nseg, d.red));
     if (split_on)
       SB_LAUNCH(d, K_EULER_Z, s,
-                k_march<R, 2, LB, WS, true, FS, true><<<gzb, MT_NT, 0, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
-                                                                  d.sc, a.rhork, a.gamrk, a.istep, slz, nsz, d.red));
+                k_march<R, 2, LB, WS, true, FS, true><<<mz.nblk, 32 * mz.nwarps, zsm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
+                                                                  d.sc, a.rhork, a.gamrk, a.istep, mz.seglen, mz.nseg, d.red));
   } else {
     SB_LAUNCH(d, K_EULER_Z, s,
-              k_march<R, 2, LB, WS, false, FS><<<gzb, MT_NT, msm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev, d.sc,
-                                                                   a.rhork, a.gamrk, a.istep, slz, nsz, d.red));
+              k_march<R, 2, LB, WS, false, FS><<<mz.nblk, 32 * mz.nwarps, zsm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev, d.sc,
+                                                                   a.rhork, a.gamrk, a.istep, mz.seglen, mz.nseg, d.red));
     if (split_on)
       SB_LAUNCH(d, K_EULER_Z, s,
-                k_march<R, 2, LB, WS, false, FS, true><<<gzb, MT_NT, 0, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
-                                                                   d.sc, a.rhork, a.gamrk, a.istep, slz, nsz, d.red));
+                k_march<R, 2, LB, WS, false, FS, true><<<mz.nblk, 32 * mz.nwarps, zsm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
+                                                                   d.sc, a.rhork, a.gamrk, a.istep, mz.seglen, mz.nseg, d.red));
   }
   if (split_on) ++*nl;
   *nl += 4;
   if (g.recyc) launch_rand_plane(g, d, s, nl);  // euler_z draws the inflow plane of the stage
   launch_bc_nr(g, d, fl_new, s, nl);
   if (g.channel_case) {
-    SB_LAUNCH(d, K_FINISH_RHS, s, k_finish_rhs<<<1, FIN_NT, 0, s>>>(g, d.red, (long long)gzb, a.istep == 1, d.sc));
+    SB_LAUNCH(d, K_FINISH_RHS, s, k_finish_rhs<<<1, FIN_NT, 0, s>>>(g, d.red, (long long)mz.nblk, a.istep == 1, d.sc));
     ++*nl;
   }
   const unsigned nbu = pt_blocks(g.nint);
