@@ -237,6 +237,8 @@ void fill_geom(streams_b200_ctx* c) {
     // the same products the reference forms in wenorec_1d (u0_2, rho0_2u0_2, ...)
     const double u0_2 = p.u0 * p.u0, r2u2 = p.rho0 * p.rho0 * u0_2, r2u4 = r2u2 * u0_2, r2u6 = r2u4 * u0_2;
     g.rcp0 = 1.0 / p.cp0;
+    g.cpp = p.cp0 / p.prandtl;
+    g.rpr = 1.0 / p.prandtl;
     g.weps_a = 0.000001 * r2u2;
     g.weps_b = 0.000001 * r2u4;
     g.weps_c = 0.000001 * r2u6;
@@ -401,6 +403,20 @@ int streams_b200_create(const streams_b200_params* p, const streams_b200_grid* g
       g.vrl[d] = dr - 1;
       g.vhl[d] = dh - 1;
       g.vrlf[d] = drf - 1;
+      std::vector<double> fr(nn[d] + 1);
+      std::vector<float> frf(nn[d] + 1);
+      for (int i = 0; i <= nn[d]; ++i) {
+        fr[i] = 1.0 / (crd[d][i + ng] - crd[d][i + ng - 1]);
+        frf[i] = static_cast<float>(fr[i]);
+      }
+      double* df;
+      float* dff;
+      if ((e = dev_alloc(c, &df, nn[d] + 1)) || (e = dev_alloc(c, &dff, nn[d] + 1))) return fail(e, "cudaMalloc(grid)");
+      if ((e = cudaMemcpy(df, fr.data(), (nn[d] + 1) * 8, cudaMemcpyHostToDevice)) ||
+          (e = cudaMemcpy(dff, frf.data(), (nn[d] + 1) * 4, cudaMemcpyHostToDevice)))
+        return fail(e, "cudaMemcpy(grid)");
+      g.vfr[d] = df;
+      g.vfrf[d] = dff;
     }
   }
   g.yn = dyn - 1;

@@ -114,22 +114,12 @@ __global__ void __launch_bounds__(XF_NT, sizeof(R) == 8 ? XF_MINB_D : XF_MINB_F)
 }
 
 template <unsigned SPAN, class R, bool TP>
-__global__ void __launch_bounds__(256, sizeof(R) == 8 ? VISC_MINB : VISC_MINB_F)
-    kb_visc(const BoxRec* __restrict__ rec, const BlockRef* __restrict__ blocks, unsigned ntile,
-    int istep, int do_sensor) {
-  for_tiles<SPAN>(rec, blocks, ntile, [&](const BoxRec* r, const Geom& g, unsigned l) {
-    d_visc<R, TP>(g, static_cast<const R*>(r->aux), fl_new_of(r, istep), static_cast<R*>(r->div3), r->sensor_next,
-                  r->wallprop, do_sensor, Blk{l, 0, 0});
-  });
-}
-
-template <unsigned SPAN, class R, bool TP>
 __global__ void __launch_bounds__(VT_NT, sizeof(R) == 8 ? VISC_MINB : VISC_MINB_F)
     kb_visc_tiled(const BoxRec* __restrict__ rec, const BlockRef* __restrict__ blocks, unsigned ntile,
     int istep, int do_sensor) {
   for_tiles<SPAN>(rec, blocks, ntile, [&](const BoxRec* r, const Geom& g, unsigned l) {
     d_visc_tiled<R, TP>(g, static_cast<const R*>(r->aux), fl_new_of(r, istep), static_cast<R*>(r->div3),
-                        r->sensor_next, r->wallprop, do_sensor, Blk{l, 0, 0});
+                        r->sensor_next, r->wallprop, do_sensor, r->vk, Blk{l, 0, 0});
   });
 }
 
@@ -247,6 +237,7 @@ cudaError_t batch_stage_impl(const BoxTable& t, const StageArgs& a, cudaStream_t
   cudaGetDevice(&dev);
   if (dev < 64 && !(smem_set & (1ULL << dev))) {
     cudaFuncSetAttribute(kb_xflux<1, R, LB, WS, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, X_SMEM_MAX);
+    cudaFuncSetAttribute(kb_visc_tiled<1, R, TP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)visc_smem<R>());
     for (auto fn : {(const void*)kb_march<1, R, 1, LB, WS, false, FS>, (const void*)kb_march<1, R, 2, LB, WS, false, FS>,
                     (const void*)kb_march<1, R, 2, LB, WS, true, FS>})
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, MARCH_SMEM_MAX);
@@ -255,11 +246,10 @@ cudaError_t batch_stage_impl(const BoxTable& t, const StageArgs& a, cudaStream_t
   const Launch X = launch_of(t, BK_X), P = launch_of(t, BK_PT);
   kb_xflux<1, R, LB, WS, FS><<<X.grid(1), dim3(XF_TX, XF_TY), XF_TY * x_warp_bytes<R, WS>(t.xslots), s>>>(t.rec, X.blocks, X.ntile, a.istep);
   const int do_sensor = fp64 && a.istep == 3;
-  if (g.conservative_viscous && SB_VISC_TILED) {
+  if (g.conservative_viscous) {
     const Launch V = launch_of(t, BK_VS);
-    kb_visc_tiled<1, R, TP><<<V.grid(1), VT_NT, 0, s>>>(t.rec, V.blocks, V.ntile, a.istep, do_sensor);
-  } else if (g.conservative_viscous)
-    kb_visc<1, R, TP><<<P.grid(1), 256, 0, s>>>(t.rec, P.blocks, P.ntile, a.istep, do_sensor);
+    kb_visc_tiled<1, R, TP><<<V.grid(1), VT_NT, visc_smem<R>(), s>>>(t.rec, V.blocks, V.ntile, a.istep, do_sensor);
+  }
   else
     kb_visc_ns<1, R, TP><<<P.grid(1), 256, 0, s>>>(t.rec, P.blocks, P.ntile, a.istep, do_sensor);
   *nl += 2;
@@ -379,6 +369,7 @@ BoxRec box_rec(const Geom& g, const DevState& d, double* fl_a, double* fl_b, dou
   r.nb_pt = nblocks(g.nint, 256);
   r.nb_vol = nblocks(g.nvol, AUX_NT);
   r.nb_vs = visc_tiled_blocks(g);
+  r.vk = visc_k(g);
   r.nb_up = pt_blocks(g.nint);
   return r;
 }

@@ -33,6 +33,9 @@ struct Geom {
   const double* vrl[3];
   const float* vrlf[3];
   const double* vhl[3];
+  // 1/(x(i+1)-x(i)) of the faces i = 0..n
+  const double* vfr[3];
+  const float* vfrf[3];
   const double* y;
   const double* z;
   const double* yn;       // yn[j], j = 1..ny+1
@@ -84,7 +87,8 @@ struct Geom {
   // 1/(rho0^2 u0^2) and 1/(rho0^2 u0^4) of wenorec_1d (kernels_cpu.F90:2539-2546) and
   // 1/(rho0^2 u0^6).  FP32 values are scaled by powers of two wsg near the square roots of those
   // scales (wsg_*i their reciprocals): wepsf = wsg^2 weps, wepsf_ab with the scale b and wsg_a
-  double gm1, rgm1, rcp0, weps_a, weps_b, weps_c;
+  double gm1, rgm1, rcp0, cpp, rpr;  // cpp = cp/Pr, rpr = 1/Pr
+  double weps_a, weps_b, weps_c;
   double wsg_a, wsg_b, wsg_c, wsg_ai, wsg_bi, wsg_ci, wepsf_a, wepsf_b, wepsf_c, wepsf_ab;
   // thermally perfect gas (calorically_perfect = 0): cp(T) = sum of cpc[l - cp_l] (T/t0)^l for
   // l = cp_l..cp_r, cv likewise (set_fluid_prop's cp_coeff / cv_coeff, times rgas0)

@@ -136,7 +136,7 @@ struct BoxRec {
   double cfl;
   int sly, nsy, slz, nsz;  // march segments (length, count) of the y and z passes
   int nwy, nwz;            // and the warps of their blocks
-  int xgrp, pad;           // x pass: groups of 32 faces a warp takes
+  int xgrp, vk;            // x pass: groups of 32 faces a warp takes; viscous pass: cells of a z segment
   unsigned nb_x, nb_vol, nb_pt, nb_y, nb_z;  // blocks of the aux pass, pointwise passes, y and z passes
   unsigned nb_vs;                      // blocks of the staged viscous pass
   unsigned nb_up;                      // blocks of the update and time-step passes

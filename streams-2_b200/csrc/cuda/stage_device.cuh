@@ -68,16 +68,10 @@ constexpr int MT_MAXW = 9, MT_SEG = 2048;
 #ifndef SB_WF_CARVEOUT
 #define SB_WF_CARVEOUT 72
 #endif
-// the viscous pass with its operands staged in shared memory (1) or read per use (0)
-#ifndef SB_VISC_TILED
-#define SB_VISC_TILED 1
-#endif
-// the viscous pass: the staged FP64 pass at 3 blocks of 256 threads per SM (80 registers; 7.42
-// against 7.57 ms per step at 4 blocks and 64 registers on the 1024x256x192 boundary layer), the
-// FP32 one at 4 (5.02 against 5.62 ms at 3); the direct pass at 4 blocks measured faster than 2
-// blocks at 128 registers
+// the viscous pass: FP64 at 2 blocks of 256 threads per SM (4.2 ms per step on the 1024x256x192
+// boundary layer; 5.8 at 3 blocks, whose 80 registers spill 140 bytes), FP32 at 4
 #ifndef VISC_MINB
-#define VISC_MINB 3
+#define VISC_MINB 2
 #endif
 // resident threads per SM asked of the register allocator for the memory-bound pointwise passes:
 // 2048 (32 registers, a little spilling in the update pass), for more loads in flight
@@ -406,6 +400,13 @@ template <class R>
 __device__ __forceinline__ R line_r(const Geom& g, int d, int i) {
   if constexpr (sizeof(R) == sizeof(double)) return __ldg(g.vrl[d] + i);
   else return __ldg(g.vrlf[d] + i);
+}
+
+// 1/(x(i+1)-x(i)) likewise, i = 0 .. n
+template <class R>
+__device__ __forceinline__ R face_r(const Geom& g, int d, int i) {
+  if constexpr (sizeof(R) == sizeof(double)) return __ldg(g.vfr[d] + i);
+  else return __ldg(g.vfrf[d] + i);
 }
 
 template <int DIR>
@@ -904,298 +905,191 @@ __global__ void __launch_bounds__(sizeof(R) == 8 ? MT_MAXT_D : MT_MAXT_F, 1) k_m
   d_march<R, DIR, LB, WS, CH, FS, SPLIT>(g, aux, sensor, fl, div3, w, fl_prev, sc, rhork, gamrk, istep, seglen, nseg, red, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
 }
 
-// visflx_reduced_ord2_subroutine (kernels_cpu.F90:4623-4721, update_sensor = 0) followed by
-// visflx_x/y/z_subroutine (:4779-4999), in the reference's accumulation order; at stage 3 also
-// sensor_subroutine (:4726-4744) into the next sensor buffer.  Arithmetic in R, accumulation
-// into the FP64 register.
-template <class R, bool TP = false>
-__device__ __forceinline__ void d_visc(const Geom& g, const R* __restrict__ aux, double* __restrict__ fl,
-                                              R* __restrict__ div3, double* __restrict__ sensor_next,
-                                              double* __restrict__ wallprop, int do_sensor, const Blk blk) {
-  const long long q = (long long)blk.x * 256 + threadIdx.x;
-  if (q >= g.nint) return;
-  int i, j, k;
-  cell_of(g, q, i, j, k);
-  const long long n = g.nvol, nI = g.nint;
-  const long long c = gidx(g, i, j, k);
-  const long long sX = 1, sY = g.sx, sZ = (long long)g.sx * g.sy;
-  auto A = [&](long long a, int m) -> R { return __ldg(aux + (m - 1) * n + a); };
-  const R uu = A(c, 2), vv = A(c, 3), ww = A(c, 4), mu = A(c, 7);
-  // cp at the point (visflx_reduced_ord2) and at a face's mean temperature (visflx_x/y/z);
-  // a constant for the calorically perfect gas
-  const R cploc = TP ? R(cp_of_t(g, double(A(c, 6)))) : R(g.cp0), prandtl = R(g.prandtl);
-  // 1/(x(i+1)-x(i-1)) etc. from the per-line tables (the same quotients as a division here)
-  R dxl, dyl, dzl;
-  if constexpr (sizeof(R) == sizeof(double)) {
-    dxl = R(__ldg(g.vrl[0] + i)); dyl = R(__ldg(g.vrl[1] + j)); dzl = R(__ldg(g.vrl[2] + k));
-  } else {
-    dxl = R(__ldg(g.vrlf[0] + i)); dyl = R(__ldg(g.vrlf[1] + j)); dzl = R(__ldg(g.vrlf[2] + k));
-  }
-  R ux = dxl * (A(c + sX, 2) - A(c - sX, 2));
-  R vx = dxl * (A(c + sX, 3) - A(c - sX, 3));
-  R wx = dxl * (A(c + sX, 4) - A(c - sX, 4));
-  R mux = dxl * (A(c + sX, 7) - A(c - sX, 7));
-  R uy = dyl * (A(c + sY, 2) - A(c - sY, 2));
-  R vy = dyl * (A(c + sY, 3) - A(c - sY, 3));
-  R wy = dyl * (A(c + sY, 4) - A(c - sY, 4));
-  R ty = dyl * (A(c + sY, 6) - A(c - sY, 6));
-  R muy = dyl * (A(c + sY, 7) - A(c - sY, 7));
-  R uz = dzl * (A(c + sZ, 2) - A(c - sZ, 2));
-  R vz = dzl * (A(c + sZ, 3) - A(c - sZ, 3));
-  R wz = dzl * (A(c + sZ, 4) - A(c - sZ, 4));
-  R muz = dzl * (A(c + sZ, 7) - A(c - sZ, 7));
-  if (j == 1) {
-    const long long wp = (long long)(k - 1) * g.nx + (i - 1);
-    const long long nw = (long long)g.nx * g.nz;
-    wallprop[wp] = double(mu * uy);
-    wallprop[nw + wp] = double(mu * wy);
-    wallprop[2 * nw + wp] = double(mu * ty * cploc / prandtl);
-  }
-  R div = ux + vy + wz;
-  R div3l = div / R(3);
-  div3[q] = div3l;
-  R omegax = wy - vz, omegay = uz - wx, omegaz = vx - uy;
-  R omod2 = omegax * omegax + omegay * omegay + omegaz * omegaz;
-  if (do_sensor) {
-    // sensor_subroutine works from the stored |omega| and div/3
-    R om = sqrt(omod2);
-    R om2 = om * om;
-    R dv = R(3) * div3l;
-    R u0l0 = R(g.u0 / g.l0);
-    R t = fmax(-dv / sqrt(om2 + dv * dv + u0l0 * u0l0), R(0));
-    sensor_next[q] = double(t * t);
-  }
-  R sig11 = ux - R(2) * div3l, sig12 = vx, sig13 = wx;
-  R sig21 = uy, sig22 = vy - R(2) * div3l, sig23 = wy;
-  R sig31 = uz, sig32 = vz, sig33 = wz - R(2) * div3l;
-  R sigx = mux * sig11 + muy * sig12 + muz * sig13;
-  R sigy = mux * sig21 + muy * sig22 + muz * sig23;
-  R sigz = mux * sig31 + muy * sig32 + muz * sig33;
-  R sigah = (sig11 * ux + sig12 * uy + sig13 * uz + sig21 * vx + sig22 * vy + sig23 * vz + sig31 * wx +
-             sig32 * wy + sig33 * wz) * mu;
-  R sigq = sigx * uu + sigy * vv + sigz * ww + sigah;
-  double f2 = fl[nI + q], f3 = fl[2 * nI + q], f4 = fl[3 * nI + q], f5 = fl[4 * nI + q];
-  f2 = f2 - double(sigx);
-  f3 = f3 - double(sigy);
-  f4 = f4 - double(sigz);
-  f5 = f5 - double(sigq);
-  // conservative face Laplacian: face sigma between points a (lower) and b (upper)
-  auto face = [&](long long a, long long b, double d, double (&s)[4]) {
-    R u1 = A(a, 2), u2 = A(b, 2), v1 = A(a, 3), v2 = A(b, 3), w1 = A(a, 4), w2 = A(b, 4);
-    R t1 = A(a, 6), t2 = A(b, 6), m1 = A(a, 7), m2 = A(b, 7);
-    R qq1 = R(0.5) * (u1 * u1 + v1 * v1 + w1 * w1);
-    R qq2 = R(0.5) * (u2 * u2 + v2 * v2 + w2 * w2);
-    R muf = m1 + m2;
-    muf = R(0.5) * muf / R(d);
-    s[0] = double((u2 - u1) * muf);
-    s[1] = double((v2 - v1) * muf);
-    s[2] = double((w2 - w1) * muf);
-    const R cpf = TP ? R(cp_of_t(g, double(R(0.5) * (t1 + t2)))) : R(g.cp0);
-    s[3] = double(((t2 - t1) * cpf / prandtl + (qq2 - qq1)) * muf);
-  };
-  double lo[4], hi[4];
-  // x: fl += dxhl*(fhat(i) - fhat(i-1)), fhat = -sigma
-  face(c - sX, c, g.x[i] - g.x[i - 1], lo);
-  face(c, c + sX, g.x[i + 1] - g.x[i], hi);
-  double dxhl = __ldg(g.vhl[0] + i);  // 2/(x(i+1)-x(i-1))
-  f2 = f2 + dxhl * (-hi[0] - -lo[0]);
-  f3 = f3 + dxhl * (-hi[1] - -lo[1]);
-  f4 = f4 + dxhl * (-hi[2] - -lo[2]);
-  f5 = f5 + dxhl * (-hi[3] - -lo[3]);
-  // y: fl = (fl + sigma(j-1/2)*dyhl) - sigma(j+1/2)*dyhl
-  face(c - sY, c, g.y[j] - g.y[j - 1], lo);
-  face(c, c + sY, g.y[j + 1] - g.y[j], hi);
-  double dyhl = __ldg(g.vhl[1] + j);
-  f2 = f2 + lo[0] * dyhl - hi[0] * dyhl;
-  f3 = f3 + lo[1] * dyhl - hi[1] * dyhl;
-  f4 = f4 + lo[2] * dyhl - hi[2] * dyhl;
-  f5 = f5 + lo[3] * dyhl - hi[3] * dyhl;
-  face(c - sZ, c, g.z[k] - g.z[k - 1], lo);
-  face(c, c + sZ, g.z[k + 1] - g.z[k], hi);
-  double dzhl = __ldg(g.vhl[2] + k);
-  f2 = f2 + lo[0] * dzhl - hi[0] * dzhl;
-  f3 = f3 + lo[1] * dzhl - hi[1] * dzhl;
-  f4 = f4 + lo[2] * dzhl - hi[2] * dzhl;
-  f5 = f5 + lo[3] * dzhl - hi[3] * dzhl;
-  fl[nI + q] = f2;
-  fl[2 * nI + q] = f3;
-  fl[3 * nI + q] = f4;
-  fl[4 * nI + q] = f5;
-}
-// The same viscous pass with its operands staged in shared memory: a block of 32 x 8 threads
-// owns a 32 x 8 column of cells and marches VT_K cells along z; the five fields the pass reads
-// (u, v, w, T, mu) of the planes k-1, k, k+1 sit in a ring of three tiles of 34 x 10 points (the
-// column and its x / y halo), so that every point is loaded once per block (and its halo once
-// more) with coalesced rows instead of once per use, and the x / y / z neighbours come from
-// shared memory.  The arithmetic is d_visc's, in its order.
-#ifndef SB_VT_K
-#define SB_VT_K 16
-#endif
-constexpr int VT_X = 32, VT_Y = 8, VT_NT = VT_X * VT_Y, VT_K = SB_VT_K;
+// The viscous pass: visflx_reduced_ord2_subroutine (kernels_cpu.F90:4623-4721, update_sensor = 0)
+// followed by visflx_x/y/z_subroutine (:4779-4999); at stage 3 also sensor_subroutine (:4726-4744)
+// into the next sensor buffer.  Arithmetic in R, accumulation into the FP64 register.
+// A block of 32 x 8 threads owns a 32 x 8 column of cells and marches vk cells along z; the five
+// fields the pass reads (u, v, w, T, mu) sit in a ring of four tiles of 34 x 10 points (the column and
+// its x / y halo): the planes k-1, k, k+1 that the cells of plane k read, and k+2, which is copied
+// (cp.async, with the cells' fl of the next plane) while plane k is computed.  Every point is loaded
+// once per block, the x / y / z neighbours come from shared memory, the flux of a cell's upper z face
+// is the next cell's lower one, and the grid's and the gas's quotients come from tables and constants
+// of the context: of the divisions of a cell (6 by face distances, 6 by the Prandtl number, one by
+// 3) none is left.
+// 1024x256x192 boundary layer, FP64: 7.4 -> 4.2 ms per step (its 112 algorithmic bytes a cell take
+// 2.5 at the copy rate); 1024x256x128 mixed: 3.4 -> 1.96; a 32x24x16 channel, whose segments were
+// 16 cells: 57 -> 9 us a pass.
+constexpr int VT_X = 32, VT_Y = 8, VT_NT = VT_X * VT_Y, VT_KMAX = 16;
 constexpr int VT_PX = VT_X + 2, VT_PY = VT_Y + 2, VT_PP = VT_PX * VT_PY;
-// blocks of the staged viscous pass: 32 x 8 columns x segments of VT_K cells in z
+template <class R>
+constexpr size_t visc_smem() { return (size_t)VT_NT * 4 * 8 + (size_t)4 * 5 * VT_PP * sizeof(R); }
+// blocks: 32 x 8 columns x segments of vk cells in z, VT_KMAX of them (two more planes are loaded per
+// segment) or fewer where that leaves SMs without their three blocks
+inline int visc_k(const Geom& g) {
+  const long long tiles = (long long)((g.nx + VT_X - 1) / VT_X) * ((g.ny + VT_Y - 1) / VT_Y);
+  return (int)std::min<long long>(VT_KMAX, std::max<long long>(1, tiles * g.nz / (148 * 3)));
+}
 inline unsigned visc_tiled_blocks(const Geom& g) {
-  return (unsigned)((g.nx + VT_X - 1) / VT_X) * (unsigned)((g.ny + VT_Y - 1) / VT_Y) *
-         (unsigned)((g.nz + VT_K - 1) / VT_K);
+  const int vk = visc_k(g);
+  return (unsigned)((g.nx + VT_X - 1) / VT_X) * (unsigned)((g.ny + VT_Y - 1) / VT_Y) * (unsigned)((g.nz + vk - 1) / vk);
 }
 template <class R, bool TP = false>
 __device__ __forceinline__ void d_visc_tiled(const Geom& g, const R* __restrict__ aux, double* __restrict__ fl,
                                              R* __restrict__ div3, double* __restrict__ sensor_next,
-                                             double* __restrict__ wallprop, int do_sensor, const Blk blk) {
-  __shared__ R pl[3][5][VT_PP];
+                                             double* __restrict__ wallprop, int do_sensor, int vk, const Blk blk) {
+  extern __shared__ __align__(16) unsigned char sb_dyn_smem[];
+  double* flb = reinterpret_cast<double*>(sb_dyn_smem) + threadIdx.x;  // this thread's fl(2:5), VT_NT apart
+  R* pl = reinterpret_cast<R*>(sb_dyn_smem + VT_NT * 4 * 8);           // [4][5][VT_PP]
   const unsigned nbx = (unsigned)(g.nx + VT_X - 1) / VT_X, nby = (unsigned)(g.ny + VT_Y - 1) / VT_Y;
   const unsigned bx = blk.x % nbx, rest = blk.x / nbx, by = rest % nby, bk = rest / nby;
   const int tx = (int)threadIdx.x % VT_X, ty = (int)threadIdx.x / VT_X;
   const int i0 = (int)bx * VT_X, j0 = (int)by * VT_Y;  // the tile's points are i0 .. i0+VT_X+1
   const int i = i0 + 1 + tx, j = j0 + 1 + ty;
   const bool own = i <= g.nx && j <= g.ny;
-  const int k0 = (int)bk * VT_K + 1, k1 = min(k0 + VT_K - 1, g.nz);
-  const long long n = g.nvol, nI = g.nint;
-  // plane k of the tile into slot k % 3 (points beyond the face ghosts are left unread: no cell
-  // of the column uses them)
+  const int k0 = (int)bk * vk + 1, k1 = min(k0 + vk - 1, g.nz);
+  const long long n = g.nvol, nI = g.nint, sZ = (long long)g.sx * g.sy, cz = (long long)g.nx * g.ny;
+  // this thread's points of a tile: t = threadIdx.x and t + VT_NT (points beyond the face ghosts are
+  // left unread: no cell of the column uses them)
+  const int t1 = threadIdx.x + VT_NT;
+  const int ia = i0 + (int)threadIdx.x % VT_PX, ja = j0 + (int)threadIdx.x / VT_PX;
+  const int ib = i0 + t1 % VT_PX, jb = j0 + t1 / VT_PX;
+  const bool ga = ia <= g.nx + 1 && ja <= g.ny + 1, gb = t1 < VT_PP && ib <= g.nx + 1 && jb <= g.ny + 1;
+  const R* pa = aux + n + gidx(g, ia, ja, 0);
+  const long long dab = gidx(g, ib, jb, 0) - gidx(g, ia, ja, 0);
+  const unsigned da = (unsigned)__cvta_generic_to_shared(pl + threadIdx.x);
   auto load_plane = [&](int k) {
-    R(*dst)[VT_PP] = pl[k % 3];
-    for (int t = threadIdx.x; t < VT_PP; t += VT_NT) {
-      const int ii = i0 + t % VT_PX, jj = j0 + t / VT_PX;
-      if (ii <= g.nx + 1 && jj <= g.ny + 1) {
-        const long long a = gidx(g, ii, jj, k);
-        dst[0][t] = __ldg(aux + n + a);
-        dst[1][t] = __ldg(aux + 2 * n + a);
-        dst[2][t] = __ldg(aux + 3 * n + a);
-        dst[3][t] = __ldg(aux + 5 * n + a);
-        dst[4][t] = __ldg(aux + 6 * n + a);
-      }
+    const unsigned d = da + (k & 3) * (unsigned)(5 * VT_PP * sizeof(R));
+    const R* s = pa + k * sZ;
+#pragma unroll
+    for (int f = 0; f < 5; ++f) {  // u, v, w, T, mu
+      const R* q = s + (f < 3 ? f : f + 1) * n;
+      if (ga) copy_async(d + f * (unsigned)(VT_PP * sizeof(R)), q);
+      if (gb) copy_async(d + (f * VT_PP + VT_NT) * (unsigned)sizeof(R), q + dab);
     }
+  };
+  const long long q0 = own ? iidx(g, i, j, 0) : 0;  // interior index of the column's plane 0
+  auto load_fl = [&](int k) {
+    if (own)
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+        copy_async((unsigned)__cvta_generic_to_shared(flb + m * VT_NT), fl + (m + 1) * nI + q0 + k * cz);
   };
   load_plane(k0 - 1);
   load_plane(k0);
-  const R prandtl = R(g.prandtl);
-  R dxl = R(0), dyl = R(0);
-  if (own) {
-    if constexpr (sizeof(R) == sizeof(double)) {
-      dxl = R(__ldg(g.vrl[0] + i)); dyl = R(__ldg(g.vrl[1] + j));
-    } else {
-      dxl = R(__ldg(g.vrlf[0] + i)); dyl = R(__ldg(g.vrlf[1] + j));
-    }
-  }
+  load_plane(k0 + 1);
+  load_fl(k0);
+  copy_commit();
+  const R cpp = TP ? R(0) : R(g.cpp), rpr = R(g.rpr);
+  R zlo[4] = {R(0), R(0), R(0), R(0)};  // flux of the lower z face
   for (int k = k0; k <= k1; ++k) {
-    load_plane(k + 1);
-    __syncthreads();
+    copy_wait<0>();
+    __syncthreads();  // plane k+1 is there, and every thread is done with plane k-2
+    double f2 = flb[0], f3 = flb[VT_NT], f4 = flb[2 * VT_NT], f5 = flb[3 * VT_NT];
+    if (k < k1) {
+      load_plane(k + 2);
+      load_fl(k + 1);
+    }
+    copy_commit();
     if (own) {
-      const int sm = (k - 1) % 3, s0 = k % 3, sp = (k + 1) % 3;
-      const int c0 = (tx + 1) + (ty + 1) * VT_PX;
-      // field f (0 u, 1 v, 2 w, 3 T, 4 mu) at the cell's point offset by (di, dj) in plane slot sl
-      auto F = [&](int sl, int di, int dj, int f) -> R { return pl[sl][f][c0 + di + dj * VT_PX]; };
-      const long long q = iidx(g, i, j, k);
-      const R uu = F(s0, 0, 0, 0), vv = F(s0, 0, 0, 1), ww = F(s0, 0, 0, 2), mu = F(s0, 0, 0, 4);
-      const R cploc = TP ? R(cp_of_t(g, double(F(s0, 0, 0, 3)))) : R(g.cp0);
-      R dzl;
-      if constexpr (sizeof(R) == sizeof(double)) dzl = R(__ldg(g.vrl[2] + k));
-      else dzl = R(__ldg(g.vrlf[2] + k));
-      R ux = dxl * (F(s0, 1, 0, 0) - F(s0, -1, 0, 0));
-      R vx = dxl * (F(s0, 1, 0, 1) - F(s0, -1, 0, 1));
-      R wx = dxl * (F(s0, 1, 0, 2) - F(s0, -1, 0, 2));
-      R mux = dxl * (F(s0, 1, 0, 4) - F(s0, -1, 0, 4));
-      R uy = dyl * (F(s0, 0, 1, 0) - F(s0, 0, -1, 0));
-      R vy = dyl * (F(s0, 0, 1, 1) - F(s0, 0, -1, 1));
-      R wy = dyl * (F(s0, 0, 1, 2) - F(s0, 0, -1, 2));
-      R ty_ = dyl * (F(s0, 0, 1, 3) - F(s0, 0, -1, 3));
-      R muy = dyl * (F(s0, 0, 1, 4) - F(s0, 0, -1, 4));
-      R uz = dzl * (F(sp, 0, 0, 0) - F(sm, 0, 0, 0));
-      R vz = dzl * (F(sp, 0, 0, 1) - F(sm, 0, 0, 1));
-      R wz = dzl * (F(sp, 0, 0, 2) - F(sm, 0, 0, 2));
-      R muz = dzl * (F(sp, 0, 0, 4) - F(sm, 0, 0, 4));
+      const R* pm = pl + ((k - 1) & 3) * 5 * VT_PP + (tx + 1) + (ty + 1) * VT_PX;
+      const R* p0 = pl + (k & 3) * 5 * VT_PP + (tx + 1) + (ty + 1) * VT_PX;
+      const R* pp = pl + ((k + 1) & 3) * 5 * VT_PP + (tx + 1) + (ty + 1) * VT_PX;
+      // field f (0 u, 1 v, 2 w, 3 T, 4 mu) at the point o of a plane
+      auto F = [&](const R* p, int o, int f) -> R { return p[f * VT_PP + o]; };
+      const long long q = q0 + k * cz;
+      const R dxl = line_r<R>(g, 0, i), dyl = line_r<R>(g, 1, j), dzl = line_r<R>(g, 2, k);
+      const R c0[5] = {F(p0, 0, 0), F(p0, 0, 1), F(p0, 0, 2), F(p0, 0, 3), F(p0, 0, 4)};
+      const R qc = R(0.5) * (c0[0] * c0[0] + c0[1] * c0[1] + c0[2] * c0[2]);
+      // conservative face Laplacian: flux at the face between the cell and its neighbour o of plane
+      // p at distance 1/rd, for the cell below (sgn = 1) or above (-1) the face
+      auto face = [&](const R* p, int o, R rd, R sgn, R (&s)[4]) {
+        const R u = F(p, o, 0), v = F(p, o, 1), w = F(p, o, 2), t = F(p, o, 3);
+        const R muf = (R(0.5) * (F(p, o, 4) + c0[4])) * (rd * sgn);
+        const R qn = R(0.5) * (u * u + v * v + w * w);
+        s[0] = (u - c0[0]) * muf;
+        s[1] = (v - c0[1]) * muf;
+        s[2] = (w - c0[2]) * muf;
+        const R cpf = TP ? R(cp_of_t(g, double(R(0.5) * (t + c0[3])))) * rpr : cpp;
+        s[3] = ((t - c0[3]) * cpf + (qn - qc)) * muf;
+      };
+      R lo[4], hi[4];
+      // x: fl += dxhl*(fhat(i) - fhat(i-1)), fhat = -sigma
+      face(p0, -1, face_r<R>(g, 0, i - 1), R(-1), lo);
+      face(p0, 1, face_r<R>(g, 0, i), R(1), hi);
+      const double dxhl = __ldg(g.vhl[0] + i);
+      f2 = f2 + dxhl * double(lo[0] - hi[0]);
+      f3 = f3 + dxhl * double(lo[1] - hi[1]);
+      f4 = f4 + dxhl * double(lo[2] - hi[2]);
+      f5 = f5 + dxhl * double(lo[3] - hi[3]);
+      face(p0, -VT_PX, face_r<R>(g, 1, j - 1), R(-1), lo);
+      face(p0, VT_PX, face_r<R>(g, 1, j), R(1), hi);
+      const double dyhl = __ldg(g.vhl[1] + j);
+      f2 = f2 + dyhl * double(lo[0] - hi[0]);
+      f3 = f3 + dyhl * double(lo[1] - hi[1]);
+      f4 = f4 + dyhl * double(lo[2] - hi[2]);
+      f5 = f5 + dyhl * double(lo[3] - hi[3]);
+      if (k == k0) face(pm, 0, face_r<R>(g, 2, k - 1), R(-1), zlo);
+      face(pp, 0, face_r<R>(g, 2, k), R(1), hi);
+      const double dzhl = __ldg(g.vhl[2] + k);
+      f2 = f2 + dzhl * double(zlo[0] - hi[0]);
+      f3 = f3 + dzhl * double(zlo[1] - hi[1]);
+      f4 = f4 + dzhl * double(zlo[2] - hi[2]);
+      f5 = f5 + dzhl * double(zlo[3] - hi[3]);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) zlo[m] = hi[m];
+      // reduced second-order terms
+      R ux = dxl * (F(p0, 1, 0) - F(p0, -1, 0));
+      R vx = dxl * (F(p0, 1, 1) - F(p0, -1, 1));
+      R wx = dxl * (F(p0, 1, 2) - F(p0, -1, 2));
+      R mux = dxl * (F(p0, 1, 4) - F(p0, -1, 4));
+      R uy = dyl * (F(p0, VT_PX, 0) - F(p0, -VT_PX, 0));
+      R vy = dyl * (F(p0, VT_PX, 1) - F(p0, -VT_PX, 1));
+      R wy = dyl * (F(p0, VT_PX, 2) - F(p0, -VT_PX, 2));
+      R muy = dyl * (F(p0, VT_PX, 4) - F(p0, -VT_PX, 4));
+      R uz = dzl * (F(pp, 0, 0) - F(pm, 0, 0));
+      R vz = dzl * (F(pp, 0, 1) - F(pm, 0, 1));
+      R wz = dzl * (F(pp, 0, 2) - F(pm, 0, 2));
+      R muz = dzl * (F(pp, 0, 4) - F(pm, 0, 4));
       if (j == 1) {
+        const R ty_ = dyl * (F(p0, VT_PX, 3) - F(p0, -VT_PX, 3));
+        const R cploc = TP ? R(cp_of_t(g, double(c0[3]))) : R(g.cp0);
         const long long wp = (long long)(k - 1) * g.nx + (i - 1);
         const long long nw = (long long)g.nx * g.nz;
-        wallprop[wp] = double(mu * uy);
-        wallprop[nw + wp] = double(mu * wy);
-        wallprop[2 * nw + wp] = double(mu * ty_ * cploc / prandtl);
+        wallprop[wp] = double(c0[4] * uy);
+        wallprop[nw + wp] = double(c0[4] * wy);
+        wallprop[2 * nw + wp] = double(c0[4] * ty_ * cploc / R(g.prandtl));
       }
-      R div = ux + vy + wz;
-      R div3l = div / R(3);
+      const R div3l = (ux + vy + wz) * R(1.0 / 3.0);
       div3[q] = div3l;
-      R omegax = wy - vz, omegay = uz - wx, omegaz = vx - uy;
-      R omod2 = omegax * omegax + omegay * omegay + omegaz * omegaz;
       if (do_sensor) {
-        R om = sqrt(omod2);
-        R om2 = om * om;
-        R dv = R(3) * div3l;
-        R u0l0 = R(g.u0 / g.l0);
-        R t = fmax(-dv / sqrt(om2 + dv * dv + u0l0 * u0l0), R(0));
+        // sensor_subroutine works from the stored |omega| and div/3
+        const R omegax = wy - vz, omegay = uz - wx, omegaz = vx - uy;
+        const R om = sqrt(omegax * omegax + omegay * omegay + omegaz * omegaz);
+        const R om2 = om * om;
+        const R dv = R(3) * div3l;
+        const R u0l0 = R(g.u0 / g.l0);
+        const R t = fmax(-dv / sqrt(om2 + dv * dv + u0l0 * u0l0), R(0));
         sensor_next[q] = double(t * t);
       }
-      R sig11 = ux - R(2) * div3l, sig12 = vx, sig13 = wx;
-      R sig21 = uy, sig22 = vy - R(2) * div3l, sig23 = wy;
-      R sig31 = uz, sig32 = vz, sig33 = wz - R(2) * div3l;
-      R sigx = mux * sig11 + muy * sig12 + muz * sig13;
-      R sigy = mux * sig21 + muy * sig22 + muz * sig23;
-      R sigz = mux * sig31 + muy * sig32 + muz * sig33;
-      R sigah = (sig11 * ux + sig12 * uy + sig13 * uz + sig21 * vx + sig22 * vy + sig23 * vz + sig31 * wx +
-                 sig32 * wy + sig33 * wz) * mu;
-      R sigq = sigx * uu + sigy * vv + sigz * ww + sigah;
-      double f2 = fl[nI + q], f3 = fl[2 * nI + q], f4 = fl[3 * nI + q], f5 = fl[4 * nI + q];
-      f2 = f2 - double(sigx);
-      f3 = f3 - double(sigy);
-      f4 = f4 - double(sigz);
-      f5 = f5 - double(sigq);
-      // conservative face Laplacian: face sigma between points a (lower) and b (upper)
-      auto face = [&](int sla, int dia, int dja, int slb, int dib, int djb, double d, double (&sf)[4]) {
-        R u1 = F(sla, dia, dja, 0), u2 = F(slb, dib, djb, 0), v1 = F(sla, dia, dja, 1), v2 = F(slb, dib, djb, 1);
-        R w1 = F(sla, dia, dja, 2), w2 = F(slb, dib, djb, 2);
-        R t1 = F(sla, dia, dja, 3), t2 = F(slb, dib, djb, 3), m1 = F(sla, dia, dja, 4), m2 = F(slb, dib, djb, 4);
-        R qq1 = R(0.5) * (u1 * u1 + v1 * v1 + w1 * w1);
-        R qq2 = R(0.5) * (u2 * u2 + v2 * v2 + w2 * w2);
-        R muf = m1 + m2;
-        muf = R(0.5) * muf / R(d);
-        sf[0] = double((u2 - u1) * muf);
-        sf[1] = double((v2 - v1) * muf);
-        sf[2] = double((w2 - w1) * muf);
-        const R cpf = TP ? R(cp_of_t(g, double(R(0.5) * (t1 + t2)))) : R(g.cp0);
-        sf[3] = double(((t2 - t1) * cpf / prandtl + (qq2 - qq1)) * muf);
-      };
-      double lo[4], hi[4];
-      face(s0, -1, 0, s0, 0, 0, g.x[i] - g.x[i - 1], lo);
-      face(s0, 0, 0, s0, 1, 0, g.x[i + 1] - g.x[i], hi);
-      double dxhl = __ldg(g.vhl[0] + i);
-      f2 = f2 + dxhl * (-hi[0] - -lo[0]);
-      f3 = f3 + dxhl * (-hi[1] - -lo[1]);
-      f4 = f4 + dxhl * (-hi[2] - -lo[2]);
-      f5 = f5 + dxhl * (-hi[3] - -lo[3]);
-      face(s0, 0, -1, s0, 0, 0, g.y[j] - g.y[j - 1], lo);
-      face(s0, 0, 0, s0, 0, 1, g.y[j + 1] - g.y[j], hi);
-      double dyhl = __ldg(g.vhl[1] + j);
-      f2 = f2 + lo[0] * dyhl - hi[0] * dyhl;
-      f3 = f3 + lo[1] * dyhl - hi[1] * dyhl;
-      f4 = f4 + lo[2] * dyhl - hi[2] * dyhl;
-      f5 = f5 + lo[3] * dyhl - hi[3] * dyhl;
-      face(sm, 0, 0, s0, 0, 0, g.z[k] - g.z[k - 1], lo);
-      face(s0, 0, 0, sp, 0, 0, g.z[k + 1] - g.z[k], hi);
-      double dzhl = __ldg(g.vhl[2] + k);
-      f2 = f2 + lo[0] * dzhl - hi[0] * dzhl;
-      f3 = f3 + lo[1] * dzhl - hi[1] * dzhl;
-      f4 = f4 + lo[2] * dzhl - hi[2] * dzhl;
-      f5 = f5 + lo[3] * dzhl - hi[3] * dzhl;
-      fl[nI + q] = f2;
-      fl[2 * nI + q] = f3;
-      fl[3 * nI + q] = f4;
-      fl[4 * nI + q] = f5;
+      const R d2 = R(2) * div3l;
+      const R sig11 = ux - d2, sig22 = vy - d2, sig33 = wz - d2;
+      const R sigx = mux * sig11 + muy * vx + muz * wx;
+      const R sigy = mux * uy + muy * sig22 + muz * wy;
+      const R sigz = mux * uz + muy * vz + muz * sig33;
+      const R sigah = (sig11 * ux + sig22 * vy + sig33 * wz + R(2) * (vx * uy + wx * uz + wy * vz)) * c0[4];
+      const R sigq = sigx * c0[0] + sigy * c0[1] + sigz * c0[2] + sigah;
+      fl[nI + q] = f2 - double(sigx);
+      fl[2 * nI + q] = f3 - double(sigy);
+      fl[3 * nI + q] = f4 - double(sigz);
+      fl[4 * nI + q] = f5 - double(sigq);
     }
-    __syncthreads();  // the slot of plane k-1 is overwritten by plane k+2 next
   }
 }
 template <class R, bool TP = false>
 __global__ void __launch_bounds__(VT_NT, sizeof(R) == 8 ? VISC_MINB : VISC_MINB_F)
     k_visc_tiled(Geom g, const R* __restrict__ aux, double* __restrict__ fl, R* __restrict__ div3,
-                 double* __restrict__ sensor_next, double* __restrict__ wallprop, int do_sensor) {
-  d_visc_tiled<R, TP>(g, aux, fl, div3, sensor_next, wallprop, do_sensor, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
-}
-
-template <class R, bool TP = false>
-__global__ void __launch_bounds__(256, sizeof(R) == 8 ? VISC_MINB : VISC_MINB_F) k_visc(Geom g, const R* __restrict__ aux, double* __restrict__ fl,
-                                              R* __restrict__ div3, double* __restrict__ sensor_next,
-                                              double* __restrict__ wallprop, int do_sensor) {
-  d_visc<R, TP>(g, aux, fl, div3, sensor_next, wallprop, do_sensor, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
+                 double* __restrict__ sensor_next, double* __restrict__ wallprop, int do_sensor, int vk) {
+  d_visc_tiled<R, TP>(g, aux, fl, div3, sensor_next, wallprop, do_sensor, vk, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
 }
 
 // visflx_nosensor_subroutine (kernels_cpu.F90:3996-4180), the non-conservative viscous form of

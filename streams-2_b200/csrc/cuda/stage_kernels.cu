@@ -168,6 +168,7 @@ static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, do
   cudaGetDevice(&dev);
   if (dev < 64 && !(smem_set & (1ULL << dev))) {
     cudaFuncSetAttribute(k_xflux<R, LB, WS, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, X_SMEM_MAX);
+    cudaFuncSetAttribute(k_visc_tiled<R, (FS & 2) != 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)visc_smem<R>());
     // block sizes and segments vary with the box: the most any takes
     for (auto fn : {(const void*)k_march<R, 1, LB, WS, false, FS>, (const void*)k_march<R, 2, LB, WS, false, FS>,
                     (const void*)k_march<R, 2, LB, WS, true, FS>, (const void*)k_march<R, 1, LB, WS, false, FS, true>,
@@ -212,14 +213,10 @@ static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, do
     ++*nl;
   }
   SB_LAUNCH(d, K_EULER_X, s, k_xflux<R, LB, WS, FS><<<xs.nblk, xb, xsm, s>>>(g, aux, sensor, fl_new, xs.ngrp));
-  if (g.conservative_viscous && SB_VISC_TILED)
+  if (g.conservative_viscous)
     SB_LAUNCH(d, K_VISC, s,
-              k_visc_tiled<R, (FS & 2) != 0><<<visc_tiled_blocks(g), VT_NT, 0, s>>>(
-                  g, aux, fl_new, div3, sensor_next, d.wallprop, fp64 && a.istep == 3));
-  else if (g.conservative_viscous)
-    SB_LAUNCH(d, K_VISC, s,
-              k_visc<R, (FS & 2) != 0><<<nblocks(g.nint, 256), 256, 0, s>>>(g, aux, fl_new, div3, sensor_next, d.wallprop,
-                                                             fp64 && a.istep == 3));
+              k_visc_tiled<R, (FS & 2) != 0><<<visc_tiled_blocks(g), VT_NT, visc_smem<R>(), s>>>(
+                  g, aux, fl_new, div3, sensor_next, d.wallprop, fp64 && a.istep == 3, visc_k(g)));
   else
     SB_LAUNCH(d, K_VISC, s,
               k_visc_ns<R, (FS & 2) != 0><<<nblocks(g.nint, 256), 256, 0, s>>>(g, aux, fl_new, div3, sensor_next, d.wallprop,
