@@ -237,6 +237,8 @@ void fill_geom(streams_b200_ctx* c) {
     // the same products the reference forms in wenorec_1d (u0_2, rho0_2u0_2, ...)
     const double u0_2 = p.u0 * p.u0, r2u2 = p.rho0 * p.rho0 * u0_2, r2u4 = r2u2 * u0_2, r2u6 = r2u4 * u0_2;
     g.rcp0 = 1.0 / p.cp0;
+    g.rcv0 = 1.0 / p.cv0;
+    g.rt0 = 1.0 / p.t0;
     g.cpp = p.cp0 / p.prandtl;
     g.rpr = 1.0 / p.prandtl;
     g.weps_a = 0.000001 * r2u2;
@@ -618,10 +620,11 @@ static int do_compute_dt(streams_b200_ctx* c) {
     return STREAMS_B200_OK;
   }
   if (!c->aux_current || c->shift_pending) {
-    SB_CHECK(c, launch_aux(c->g, c->d, c->shift_pending ? 1 : 0, c->stream, &c->launches));
+    SB_CHECK(c, launch_aux_dt(c->g, c->d, c->shift_pending ? 1 : 0, c->p.cfl, c->stream, &c->launches));
     c->shift_pending = false;
     c->aux_current = true;
     c->stats_ready = false;
+    return STREAMS_B200_OK;
   }
   SB_CHECK(c, launch_dt(c->g, c->d, c->p.cfl, c->stream, &c->launches));
   return STREAMS_B200_OK;
@@ -1152,15 +1155,16 @@ int group_step(streams_b200_batch* b, const BatchBranch& br, long long step, cud
   cudaError_t e = cudaSuccess;
   if (c0->p.cfl > 0 && step % b->dt_every == 0) {
     if (!c0->aux_current || c0->shift_pending) {
-      e = batch_launch_aux(t, c0->shift_pending ? 1 : 0, s, &nl);
+      e = batch_launch_aux_dt(t, c0->shift_pending ? 1 : 0, s, &nl);
       for (int q : br.boxes) {
         streams_b200_ctx* c = b->ctxs[q];
         c->shift_pending = false;
         c->aux_current = true;
         c->stats_ready = false;
       }
+    } else {
+      e = batch_launch_dt(t, s, &nl);
     }
-    if (e == cudaSuccess) e = batch_launch_dt(t, s, &nl);
   }
   const bool fv = c0->g.force_var != 0;
   for (int istep = 1; istep <= 3 && e == cudaSuccess; ++istep) {

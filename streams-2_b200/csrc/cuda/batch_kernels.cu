@@ -97,11 +97,11 @@ __global__ void __launch_bounds__(AUX_NT) kb_apply_shift(const BoxRec* __restric
   });
 }
 
-template <unsigned SPAN, class A, bool TP>
-__global__ void __launch_bounds__(AUX_NT, AUX_MINB) kb_aux(const BoxRec* __restrict__ rec,
+template <unsigned SPAN, class A, bool TP, bool DT>
+__global__ void __launch_bounds__(AUX_NT, DT ? AUX_MINB_DT : AUX_MINB) kb_aux(const BoxRec* __restrict__ rec,
     const BlockRef* __restrict__ blocks, unsigned ntile, int want_vel) {
   for_tiles<SPAN>(rec, blocks, ntile, [&](const BoxRec* r, const Geom& g, unsigned l) {
-    d_aux<A, TP>(g, r->w, static_cast<A*>(r->aux), 0, want_vel ? r->vel64 : nullptr, Blk{l, 0, 0});
+    d_aux<A, TP, DT>(g, r->w, static_cast<A*>(r->aux), 0, want_vel ? r->vel64 : nullptr, r->red, Blk{l, 0, 0});
   });
 }
 
@@ -186,9 +186,9 @@ __global__ void __launch_bounds__(256, DT_MINB) kb_dt(const BoxRec* __restrict__
   });
 }
 
-__global__ void __launch_bounds__(FIN_NT) kb_dt_finish(const BoxRec* __restrict__ rec) {
+__global__ void __launch_bounds__(FIN_NT) kb_dt_finish(const BoxRec* __restrict__ rec, int from_aux) {
   const BoxRec* r = rec + blockIdx.x;
-  d_dt_finish(r->red, r->nb_up, r->cfl, r->sc, Blk{0, 0, 0});
+  d_dt_finish(r->red, from_aux ? r->nb_vol : r->nb_up, r->cfl, r->sc, Blk{0, 0, 0});
 }
 
 // Tiles per CTA: the short tiles of the aux, shift and sensor passes are taken four at a time so
@@ -203,26 +203,27 @@ struct Launch {
 inline Launch launch_of(const BoxTable& t, int kind) { return Launch{t.cnt[kind], t.blocks + t.off[kind]}; }
 
 template <class R, bool TP>
-void batch_aux_tp(const BoxTable& t, int apply_shift, int want_vel, cudaStream_t s, long long* nl) {
+void batch_aux_tp(const BoxTable& t, int apply_shift, int want_vel, bool dt, cudaStream_t s, long long* nl) {
   if (apply_shift) {
     const Launch L = launch_of(t, BK_PT);
     kb_apply_shift<SPAN_PT, R, TP><<<L.grid(SPAN_PT), AUX_NT, 0, s>>>(t.rec, L.blocks, L.ntile);
     ++*nl;
   }
   const Launch L = launch_of(t, BK_VOL);
-  kb_aux<SPAN_PT, R, TP><<<L.grid(SPAN_PT), AUX_NT, 0, s>>>(t.rec, L.blocks, L.ntile, want_vel);
+  if (dt) kb_aux<SPAN_PT, R, TP, true><<<L.grid(SPAN_PT), AUX_NT, 0, s>>>(t.rec, L.blocks, L.ntile, want_vel);
+  else kb_aux<SPAN_PT, R, TP, false><<<L.grid(SPAN_PT), AUX_NT, 0, s>>>(t.rec, L.blocks, L.ntile, want_vel);
   ++*nl;
 }
 
 template <class R>
-void batch_aux(const BoxTable& t, int apply_shift, int want_vel, cudaStream_t s, long long* nl) {
+void batch_aux(const BoxTable& t, int apply_shift, int want_vel, bool dt, cudaStream_t s, long long* nl) {
   if constexpr (sizeof(R) == sizeof(double)) {
     if (!t.g0.calorically_perfect) {
-      batch_aux_tp<R, true>(t, apply_shift, want_vel, s, nl);
+      batch_aux_tp<R, true>(t, apply_shift, want_vel, dt, s, nl);
       return;
     }
   }
-  batch_aux_tp<R, false>(t, apply_shift, want_vel, s, nl);
+  batch_aux_tp<R, false>(t, apply_shift, want_vel, dt, s, nl);
 }
 
 template <class R, int LB, int WS, int FS>
@@ -231,7 +232,7 @@ cudaError_t batch_stage_impl(const BoxTable& t, const StageArgs& a, cudaStream_t
   constexpr bool fp64 = sizeof(R) == sizeof(double);
   constexpr bool TP = (FS & 2) != 0;
   const int nbox = t.nbox;
-  if (a.run_aux) batch_aux<R>(t, a.apply_shift, !fp64 && a.istep == 3, s, nl);
+  if (a.run_aux) batch_aux<R>(t, a.apply_shift, !fp64 && a.istep == 3, false, s, nl);
   static unsigned long long smem_set = 0;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -440,9 +441,11 @@ cudaError_t box_table_build(BoxTable& t, const std::vector<BoxRec>& recs, cudaSt
   return cudaSuccess;
 }
 
-cudaError_t batch_launch_aux(const BoxTable& t, int apply_shift, cudaStream_t s, long long* nl) {
-  if (t.g0.precision == 1) batch_aux<float>(t, apply_shift, 0, s, nl);
-  else batch_aux<double>(t, apply_shift, 0, s, nl);
+cudaError_t batch_launch_aux_dt(const BoxTable& t, int apply_shift, cudaStream_t s, long long* nl) {
+  if (t.g0.precision == 1) batch_aux<float>(t, apply_shift, 0, true, s, nl);
+  else batch_aux<double>(t, apply_shift, 0, true, s, nl);
+  kb_dt_finish<<<t.nbox, FIN_NT, 0, s>>>(t.rec, 1);
+  ++*nl;
   return cudaGetLastError();
 }
 
@@ -452,7 +455,7 @@ cudaError_t batch_launch_dt(const BoxTable& t, cudaStream_t s, long long* nl) {
     kb_dt<1, float><<<U.grid(1), 256, 0, s>>>(t.rec, U.blocks, U.ntile);
   else
     kb_dt<1, double><<<U.grid(1), 256, 0, s>>>(t.rec, U.blocks, U.ntile);
-  kb_dt_finish<<<t.nbox, FIN_NT, 0, s>>>(t.rec);
+  kb_dt_finish<<<t.nbox, FIN_NT, 0, s>>>(t.rec, 0);
   *nl += 2;
   return cudaGetLastError();
 }

@@ -87,7 +87,7 @@ struct Geom {
   // 1/(rho0^2 u0^2) and 1/(rho0^2 u0^4) of wenorec_1d (kernels_cpu.F90:2539-2546) and
   // 1/(rho0^2 u0^6).  FP32 values are scaled by powers of two wsg near the square roots of those
   // scales (wsg_*i their reciprocals): wepsf = wsg^2 weps, wepsf_ab with the scale b and wsg_a
-  double gm1, rgm1, rcp0, cpp, rpr;  // cpp = cp/Pr, rpr = 1/Pr
+  double gm1, rgm1, rcp0, rcv0, rt0, cpp, rpr;  // 1/cp, 1/cv, 1/t0, cp/Pr, 1/Pr
   double weps_a, weps_b, weps_c;
   double wsg_a, wsg_b, wsg_c, wsg_ai, wsg_bi, wsg_ci, wepsf_a, wepsf_b, wepsf_c, wepsf_ab;
   // thermally perfect gas (calorically_perfect = 0): cp(T) = sum of cpc[l - cp_l] (T/t0)^l for
@@ -167,6 +167,27 @@ struct Scalars {
   int pad;
 };
 
+// Reciprocal and reciprocal square root in FP64: the hardware's approximation y
+// (about 20 correct bits) corrected by the first terms of the binomial series of its residual,
+//   1/b = y/(1 - e) = y (1 + e + e^2 + ..),               e = 1 - b y,
+//   1/sqrt(x) = y/sqrt(1 - e) = y (1 + e/2 + 3 e^2/8 + ..),  e = 1 - x y^2,
+// which leaves e^3 (below 2^-57) and the rounding of the last operations, about one unit in the
+// last place.  Arguments are positive and normal (densities, squared sound speeds, sums of weights).
+// They stand for the IEEE quotients and square roots, which branch for their special cases, of the
+// Roe average (three) and of the weights (one for the two sides of a field) of a WENO face, and for
+// the quotients by the density of the pointwise passes.
+__device__ __forceinline__ double rcp_pos(double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  const double e = fma(-b, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double rsqrt_pos(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
 // x^l for an integer exponent (Fortran's ** with an integer power)
 __host__ __device__ __forceinline__ double ipow_d(double x, int l) {
   double r = 1.0;
@@ -209,14 +230,14 @@ __device__ __forceinline__ double tp_newton(const Geom& g, const double* c, doub
 template <bool TPA = true>
 __device__ __forceinline__ double t_from_e(const Geom& g, double ee, double t_start) {
   double ebar = ee - g.cv_last * g.t0;
-  if (!TPA || g.calorically_perfect) return g.t0 + ebar / g.cv0;
+  if (!TPA || g.calorically_perfect) return g.t0 + ebar * g.rcv0;
   return tp_newton(g, g.cvc, ebar, t_start);
 }
 template <bool TPA = true>
 __device__ __forceinline__ double e_from_t(const Geom& g, double tt) {
   double ee = g.cv_last;
   if (!TPA || g.calorically_perfect) {
-    ee = ee + g.cv0 * (tt / g.t0 - 1.0);
+    ee = ee + g.cv0 * (tt * g.rt0 - 1.0);
   } else {
     const double tr = tt / g.t0;
     double tp = ipow_d(tr, g.cp_l + 1);  // (T/t0)^(l+1)
@@ -251,23 +272,23 @@ __device__ __forceinline__ double gamloc_of_t(const Geom& g, double tt) {
 template <bool TPA = true>
 __device__ __forceinline__ double shifted_rhoe(const Geom& g, double rho, double rhou, double rhov, double rhow,
                                                double rhoe, double tbdiff, double t_start) {
-  double ri = 1.0 / rho;
+  double ri = rcp_pos(rho);
   double uu = rhou * ri, vv = rhov * ri, ww = rhow * ri;
   double qq = 0.5 * (uu * uu + vv * vv + ww * ww);
-  double ee = rhoe / rho - qq;
+  double ee = rhoe * ri - qq;
   double tt = t_from_e<TPA>(g, ee, t_start);
   double ttnew = tt + tbdiff;
   double en = e_from_t<TPA>(g, ttnew);
-  return rho * en + 0.5 * (rhou * rhou + rhov * rhov + rhow * rhow) / rho;
+  return rho * en + 0.5 * (rhou * rhou + rhov * rhov + rhow * rhow) * ri;
 }
 
 // viscosity law of eval_aux_subroutine (kernels_cpu.F90:6995-7002)
 __device__ __forceinline__ double viscosity(const Geom& g, double tt) {
-  if (g.visc_model == 1) return g.mu0 * pow(tt / g.t0, g.vtexp);
+  if (g.visc_model == 1) return g.mu0 * pow(tt * g.rt0, g.vtexp);
   if (g.visc_model == 2) {
-    double tr = tt / g.t0;
+    double tr = tt * g.rt0;
     double st = g.sutherland_s / g.t_ref_dim;
-    return g.mu0 * pow(tr, 1.5) * (1.0 + st) / (tr + st);
+    return g.mu0 * (tr * sqrt(tr)) * (1.0 + st) / (tr + st);
   }
   return 0.0;
 }

@@ -50,27 +50,7 @@ __device__ __forceinline__ R fsqrt_pos(R x) {
   }
 }
 
-// Reciprocal and reciprocal square root in the FP64 flux arithmetic: the hardware's approximation y
-// (about 20 correct bits) corrected by the first terms of the binomial series of its residual,
-//   1/b = y/(1 - e) = y (1 + e + e^2 + ..),               e = 1 - b y,
-//   1/sqrt(x) = y/sqrt(1 - e) = y (1 + e/2 + 3 e^2/8 + ..),  e = 1 - x y^2,
-// which leaves e^3 (below 2^-57) and the rounding of the last operations, about one unit in the
-// last place.  Arguments are positive and normal (densities, squared sound speeds, sums of weights).
-// They stand for the IEEE quotients and square roots, which branch for their special cases, of the
-// Roe average (three) and of the weights (one for the two sides of a field) of a WENO face.
-__device__ __forceinline__ double rcp_pos(double b) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  const double e = fma(-b, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
 __device__ __forceinline__ float rcp_pos(float b) { return fdiv(1.0f, b); }
-__device__ __forceinline__ double rsqrt_pos(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
 __device__ __forceinline__ float rsqrt_pos(float x) { return rsqrt(x); }
 // maximum that keeps b when a is not a number (as fmax does for the running maxima here), without
 // fmax's handling of two of them in FP64

@@ -91,6 +91,8 @@ struct StageArgs {
 cudaError_t launch_aux(const Geom& g, DevState& d, int apply_shift, cudaStream_t s, long long* nl);
 cudaError_t launch_init_sensor(const Geom& g, DevState& d, cudaStream_t s, long long* nl);
 cudaError_t launch_dt(const Geom& g, DevState& d, double cfl, cudaStream_t s, long long* nl);
+// the aux pass and the time step from it
+cudaError_t launch_aux_dt(const Geom& g, DevState& d, int apply_shift, double cfl, cudaStream_t s, long long* nl);
 // One RK stage.  fl_prev holds the previous stage's right-hand side (unused at stage 1),
 // fl_new receives this stage's.  At stage 3 the next Ducros sensor becomes current.
 cudaError_t launch_stage(const Geom& g, DevState& d, const StageArgs& a, double* fl_prev, double* fl_new,
@@ -169,7 +171,7 @@ long long batch_key(const Geom& g);
 BoxRec box_rec(const Geom& g, const DevState& d, double* fl_a, double* fl_b, double cfl);
 cudaError_t box_table_build(BoxTable& t, const std::vector<BoxRec>& recs, cudaStream_t s);
 void box_table_free(BoxTable& t, cudaStream_t s);
-cudaError_t batch_launch_aux(const BoxTable& t, int apply_shift, cudaStream_t s, long long* nl);
+cudaError_t batch_launch_aux_dt(const BoxTable& t, int apply_shift, cudaStream_t s, long long* nl);
 cudaError_t batch_launch_dt(const BoxTable& t, cudaStream_t s, long long* nl);
 cudaError_t batch_launch_stage(const BoxTable& t, const StageArgs& a, cudaStream_t s, long long* nl);
 

@@ -84,6 +84,9 @@ constexpr int MT_MAXW = 9, MT_SEG = 2048;
 #ifndef AUX_MINB
 #define AUX_MINB 8
 #endif
+#ifndef AUX_MINB_DT
+#define AUX_MINB_DT 6
+#endif
 #ifndef DT_MINB
 #define DT_MINB 8
 #endif
@@ -171,73 +174,108 @@ __device__ __forceinline__ void point_state(const Geom& g, const double* __restr
   st[0] = rho; st[1] = rhou; st[2] = rhov; st[3] = rhow; st[4] = rhoe;
 }
 
+// Inverse time scales of a cell (compute_dt_subroutine, kernels_cpu.F90:6814-6880): the largest of
+// the nine, three convective, three viscous and three conductive ones.  Rounding is monotone, so the
+// largest of the products with a metric is the product of the largest.
+__device__ __forceinline__ double inverse_dt(const Geom& g, int i, int j, int k, double uu, double vv, double ww,
+                                             double cs, double nu) {
+  const double kr = nu / g.prandtl, nk = fmax(nu, kr);
+  double m = fmax((fabs(uu) + cs) * g.dcsidx[i], fmax((fabs(vv) + cs) * g.detady[j], (fabs(ww) + cs) * g.dzitdz[k]));
+  return fmax(m, nk * fmax(g.dcsidxs[i], fmax(g.detadys[j], g.dzitdzs[k])));
+}
+// largest of the block's values (non-negative) into out
+__device__ __forceinline__ void block_max(double m, double* __restrict__ out) {
+  __shared__ double sm[32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < (int)(blockDim.x >> 5); ++q) m = fmax(m, sm[q]);
+    *out = m;
+  }
+}
+
 // w -> aux at all interior and face-ghost points (eval_aux_subroutine, kernels_cpu.F90:6960-7011),
 // computed in FP64 and stored as A; with write_ghost_w = 1 the ghost states are also stored into
 // w, with write_ghost_w = 2 only they are (aux is left as it is).  With vel non-null the FP64
-// velocities are stored too (the mixed form's stage-3 sensor reads them).
-template <class A, bool TP = false>
-__device__ __forceinline__ void d_aux(const Geom& g, double* __restrict__ w, A* __restrict__ aux,
-                                                int write_ghost_w, double* __restrict__ vel, const Blk blk) {
+// velocities are stored too (the mixed form's stage-3 sensor reads them).  DT: the pass that starts
+// a step also leaves the block maxima of the inverse time scales in red, for which a pass of its own
+// read 48 (FP64) or 40 (mixed) bytes a cell: 1024x256x192, both passes 4.04 -> 3.21 ms per step,
+// 1024x256x128 mixed 2.38 -> 1.76.  Memory bound (104 and 68 bytes a point); quotients by the density
+// and by constants are products with reciprocals.
+template <class A, bool TP, bool DT>
+__device__ __forceinline__ void d_aux(const Geom& g, double* __restrict__ w, A* __restrict__ aux, int write_ghost_w,
+                                      double* __restrict__ vel, double* __restrict__ red, const Blk blk) {
   const long long n = g.nvol;
   const long long q = (long long)blk.x * AUX_NT + threadIdx.x;
-  if (q >= n) return;
-  const int ii = (int)(q % g.sx);
-  const int jj = (int)((q / g.sx) % g.sy);
-  const int kk = (int)(q / ((long long)g.sx * g.sy));
-  const int i = ii - g.ng + 1, j = jj - g.ng + 1, k = kk - g.ng + 1;
-  const int ox = (i < 1 || i > g.nx), oy = (j < 1 || j > g.ny), oz = (k < 1 || k > g.nz);
-  if (ox + oy + oz > 1) return;  // halo edges and corners are never read
-  if (write_ghost_w == 2 && !(ox | oy | oz)) return;
-  const long long dst = gidx(g, i, j, k);
-  // Newton starts (thermally perfect gas): the point's previous temperature, as eval_aux starts
-  // from w_aux(6); for a wall ghost the mirror of it estimates the interior source point's
-  double t_old = g.t0, t_src = g.t0;
-  if constexpr (TP) {
-    t_old = double(aux[5 * n + dst]);
-    if (!(t_old > 0.0)) t_old = g.t0;
-    t_src = 2.0 * g.t_wall - t_old;
-    if (!(t_src > 0.0)) t_src = g.t0;
-  }
-  double st[5];
-  point_state<TP>(g, w, i, j, k, st, t_src);
-  double rho = st[0], rhou = st[1], rhov = st[2], rhow = st[3], rhoe = st[4];
-  if (write_ghost_w && (ox | oy | oz)) {
-    w[dst] = rho; w[n + dst] = rhou; w[2 * n + dst] = rhov; w[3 * n + dst] = rhow; w[4 * n + dst] = rhoe;
-  }
-  if (write_ghost_w == 2) return;  // ghost layers of w only; aux keeps its values
-  double ri = 1.0 / rho;
-  double uu = rhou * ri, vv = rhov * ri, ww = rhow * ri;
-  double qq = 0.5 * (uu * uu + vv * vv + ww * ww);
-  double ee = rhoe / rho - qq;
-  double tt = t_from_e<TP>(g, ee, t_old);
-  double pp = rho * tt * g.rgas0;
-  if (vel) {  // FP64 velocities, as the sensor forms them from w
-    vel[dst] = uu;
-    vel[n + dst] = vv;
-    vel[2 * n + dst] = ww;
-  }
-  aux[dst] = A(rho);
-  aux[n + dst] = A(uu);
-  aux[2 * n + dst] = A(vv);
-  aux[3 * n + dst] = A(ww);
-  aux[4 * n + dst] = A((rhoe + pp) / rho);
-  aux[5 * n + dst] = A(tt);
-  // the mixed form's viscous arithmetic is FP32, and so is its viscosity law (with SB_FP32_FAST)
-  if constexpr (sizeof(A) == sizeof(float) && SB_FP32_FAST != 0)
-    aux[6 * n + dst] = viscosity_f(g, float(tt));
-  else
-    aux[6 * n + dst] = A(viscosity(g, tt));
-  // FP64 form: the sound speed, which the WENO eigenvalue bound of every face reads at its
-  // stencil points (the same expression the flux would form)
-  if constexpr (sizeof(A) == sizeof(double)) {
-    const double gq = TP ? gamloc_of_t(g, tt) : g.gamloc;
-    aux[7 * n + dst] = sqrt(gq * g.rgas0 * tt);
-  }
+  double m = 0.0;
+  auto point = [&]() {
+    const unsigned qu = (unsigned)q, r = qu / (unsigned)g.sx;  // fewer than 2^32 points: more do not fit the memory
+    const int ii = (int)(qu - r * (unsigned)g.sx);
+    const int kk = (int)(r / (unsigned)g.sy), jj = (int)(r - (unsigned)kk * (unsigned)g.sy);
+    const int i = ii - g.ng + 1, j = jj - g.ng + 1, k = kk - g.ng + 1;
+    const int ox = (i < 1 || i > g.nx), oy = (j < 1 || j > g.ny), oz = (k < 1 || k > g.nz);
+    if (ox + oy + oz > 1) return;  // halo edges and corners are never read
+    if (write_ghost_w == 2 && !(ox | oy | oz)) return;
+    const long long dst = gidx(g, i, j, k);
+    // Newton starts (thermally perfect gas): the point's previous temperature, as eval_aux starts
+    // from w_aux(6); for a wall ghost the mirror of it estimates the interior source point's
+    double t_old = g.t0, t_src = g.t0;
+    if constexpr (TP) {
+      t_old = double(aux[5 * n + dst]);
+      if (!(t_old > 0.0)) t_old = g.t0;
+      t_src = 2.0 * g.t_wall - t_old;
+      if (!(t_src > 0.0)) t_src = g.t0;
+    }
+    double st[5];
+    point_state<TP>(g, w, i, j, k, st, t_src);
+    const double rho = st[0], rhou = st[1], rhov = st[2], rhow = st[3], rhoe = st[4];
+    if (write_ghost_w && (ox | oy | oz)) {
+      w[dst] = rho; w[n + dst] = rhou; w[2 * n + dst] = rhov; w[3 * n + dst] = rhow; w[4 * n + dst] = rhoe;
+    }
+    if (write_ghost_w == 2) return;  // ghost layers of w only; aux keeps its values
+    const double ri = rcp_pos(rho);
+    const double uu = rhou * ri, vv = rhov * ri, ww = rhow * ri;
+    const double qq = 0.5 * (uu * uu + vv * vv + ww * ww);
+    const double ee = rhoe * ri - qq;
+    const double tt = t_from_e<TP>(g, ee, t_old);
+    const double pp = rho * tt * g.rgas0;
+    if (vel) {  // FP64 velocities, as the sensor forms them from w
+      vel[dst] = uu;
+      vel[n + dst] = vv;
+      vel[2 * n + dst] = ww;
+    }
+    aux[dst] = A(rho);
+    aux[n + dst] = A(uu);
+    aux[2 * n + dst] = A(vv);
+    aux[3 * n + dst] = A(ww);
+    aux[4 * n + dst] = A((rhoe + pp) * ri);
+    aux[5 * n + dst] = A(tt);
+    double mu = 0.0, cs = 0.0;
+    if constexpr (DT || sizeof(A) == sizeof(double)) {
+      mu = viscosity(g, tt);
+      cs = sqrt((TP ? gamloc_of_t(g, tt) : g.gamloc) * g.rgas0 * tt);
+    }
+    // the mixed form's viscous arithmetic is FP32, and so is its viscosity law (with SB_FP32_FAST)
+    if constexpr (sizeof(A) == sizeof(float) && SB_FP32_FAST != 0)
+      aux[6 * n + dst] = viscosity_f(g, float(tt));
+    else
+      aux[6 * n + dst] = A(viscosity(g, tt));
+    // FP64 form: the sound speed, which the WENO eigenvalue bound of every face reads at its
+    // stencil points (the same expression the flux would form)
+    if constexpr (sizeof(A) == sizeof(double)) aux[7 * n + dst] = cs;
+    if constexpr (DT)
+      if (!(ox | oy | oz)) m = inverse_dt(g, i, j, k, uu, vv, ww, cs, ri * mu);
+  };
+  if (q < n) point();
+  if constexpr (DT) block_max(m, red + blk.x);
 }
-template <class A, bool TP = false>
-__global__ void __launch_bounds__(AUX_NT, AUX_MINB) k_aux(Geom g, double* __restrict__ w, A* __restrict__ aux,
-                                                int write_ghost_w, double* __restrict__ vel) {
-  d_aux<A, TP>(g, w, aux, write_ghost_w, vel, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
+template <class A, bool TP = false, bool DT = false>
+__global__ void __launch_bounds__(AUX_NT, DT ? AUX_MINB_DT : AUX_MINB)
+    k_aux(Geom g, double* __restrict__ w, A* __restrict__ aux, int write_ghost_w, double* __restrict__ vel,
+          double* __restrict__ red) {
+  d_aux<A, TP, DT>(g, w, aux, write_ghost_w, vel, red, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
 }
 
 // Ducros sensor in FP64 from w for the mixed form, so that the central/WENO switch is taken
@@ -1228,13 +1266,12 @@ __global__ void __launch_bounds__(256) k_init_sensor(Geom g, const R* __restrict
   d_init_sensor<R>(g, aux, sensor, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
 }
 
-// compute_dt_subroutine (kernels_cpu.F90:6814-6880): block maxima of the 9 inverse time scales.
-// The FP64 form reads the primitive fields; the mixed form recomputes them from w in FP64.
+// The time step where the aux pass does not run (aux is current): block maxima of the inverse time
+// scales.  The FP64 form reads the primitive fields; the mixed form recomputes them from w in FP64.
 template <class R>
 __device__ __forceinline__ void d_dt(const Geom& g, const double* __restrict__ w, const R* __restrict__ aux,
                                             double* __restrict__ red, const Blk blk) {
-  __shared__ double sm[9 * 8];
-  double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  double m = 0.0;
 #pragma unroll 1
   for (int cq = 0; cq < PT_CELLS; ++cq) {
     const long long q = (long long)blk.x * (256 * PT_CELLS) + cq * 256 + threadIdx.x;
@@ -1242,8 +1279,7 @@ __device__ __forceinline__ void d_dt(const Geom& g, const double* __restrict__ w
     int i, j, k;
     cell_of(g, q, i, j, k);
     const long long n = g.nvol, c = gidx(g, i, j, k);
-    double rho = w[c];
-    double ri = 1.0 / rho;
+    const double ri = rcp_pos(w[c]);
     double uu, vv, ww, tt, mu;
     if constexpr (sizeof(R) == sizeof(double)) {
       uu = aux[n + c]; vv = aux[2 * n + c]; ww = aux[3 * n + c]; tt = aux[5 * n + c]; mu = aux[6 * n + c];
@@ -1251,33 +1287,10 @@ __device__ __forceinline__ void d_dt(const Geom& g, const double* __restrict__ w
       const Prim p = prim_from_w<false>(g, w, c, g.t0);  // mixed form only: calorically perfect
       uu = p.uu; vv = p.vv; ww = p.ww; tt = p.tt; mu = viscosity(g, tt);
     }
-    double nu = ri * mu;
-    double kr = nu / g.prandtl;
-    double cs = sqrt(gamloc_of_t(g, tt) * g.rgas0 * tt);
-    v[0] = fmax(v[0], (fabs(uu) + cs) * g.dcsidx[i]);
-    v[1] = fmax(v[1], (fabs(vv) + cs) * g.detady[j]);
-    v[2] = fmax(v[2], (fabs(ww) + cs) * g.dzitdz[k]);
-    v[3] = fmax(v[3], nu * g.dcsidxs[i]);
-    v[4] = fmax(v[4], nu * g.detadys[j]);
-    v[5] = fmax(v[5], nu * g.dzitdzs[k]);
-    v[6] = fmax(v[6], kr * g.dcsidxs[i]);
-    v[7] = fmax(v[7], kr * g.detadys[j]);
-    v[8] = fmax(v[8], kr * g.dzitdzs[k]);
+    const double cs = sqrt(gamloc_of_t(g, tt) * g.rgas0 * tt);
+    m = fmax(m, inverse_dt(g, i, j, k, uu, vv, ww, cs, ri * mu));
   }
-#pragma unroll
-  for (int r = 0; r < 9; ++r)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[r] = fmax(v[r], __shfl_down_sync(0xffffffffu, v[r], o));
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0)
-#pragma unroll
-    for (int r = 0; r < 9; ++r) sm[r * 8 + warp] = v[r];
-  __syncthreads();
-  if (threadIdx.x < 9) {
-    double m = 0.0;
-    for (int wq = 0; wq < 8; ++wq) m = fmax(m, sm[threadIdx.x * 8 + wq]);
-    red[(long long)blk.x * 9 + threadIdx.x] = m;
-  }
+  block_max(m, red + blk.x);
 }
 template <class R>
 __global__ void __launch_bounds__(256, DT_MINB) k_dt(Geom g, const double* __restrict__ w, const R* __restrict__ aux,
@@ -1289,7 +1302,7 @@ __device__ __forceinline__ void d_dt_finish(const double* __restrict__ red, long
                                                       Scalars* __restrict__ sc, const Blk blk) {
   __shared__ double sm[FIN_NT / 32];
   double m = 0.0;
-  for (long long b = threadIdx.x; b < nblk * 9; b += FIN_NT) m = fmax(m, red[b]);
+  for (long long b = threadIdx.x; b < nblk; b += FIN_NT) m = fmax(m, red[b]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;

@@ -51,7 +51,7 @@ void Prof::reset() {
 }
 
 long long reduction_slots(const Geom& g) {
-  long long a = (long long)nblocks(g.nint, 256) * (NRED_UPD > 9 ? NRED_UPD : 9);
+  long long a = std::max((long long)nblocks(g.nint, 256) * NRED_UPD, (long long)nblocks(g.nvol, AUX_NT));
   // the largest segment count any tuning can reach: segments of MARCH_MINSEG_MIN cells
   const long long nseg = std::max(1, (g.eul_kmax - g.eul_kmin + 1 + MARCH_MINSEG_MIN - 1) / MARCH_MINSEG_MIN);
   long long b = (((long long)g.nx * g.ny + 31) / 32) * nseg * 5;
@@ -63,32 +63,44 @@ long long reduction_slots(const Geom& g) {
 // interior points as the sources of ghost states, so it must not rewrite them itself.
 template <class R, bool TP>
 static void aux_launch_tp(const Geom& g, DevState& d, int apply_shift, int write_ghost, int kid, cudaStream_t s,
-                          long long* nl, double* vel) {
+                          long long* nl, double* vel, bool dt) {
   if (apply_shift) {
     SB_LAUNCH(d, K_APPLY_SHIFT, s,
               k_apply_shift<R, TP><<<nblocks(g.nint, AUX_NT), AUX_NT, 0, s>>>(g, d.w, aux_of<R>(d), d.sc));
     ++*nl;
   }
-  SB_LAUNCH(d, kid, s,
-            k_aux<R, TP><<<nblocks(g.nvol, AUX_NT), AUX_NT, 0, s>>>(g, d.w, aux_of<R>(d), write_ghost, vel));
+  if (dt)
+    SB_LAUNCH(d, kid, s,
+              k_aux<R, TP, true><<<nblocks(g.nvol, AUX_NT), AUX_NT, 0, s>>>(g, d.w, aux_of<R>(d), write_ghost, vel, d.red));
+  else
+    SB_LAUNCH(d, kid, s,
+              k_aux<R, TP><<<nblocks(g.nvol, AUX_NT), AUX_NT, 0, s>>>(g, d.w, aux_of<R>(d), write_ghost, vel, nullptr));
   ++*nl;
 }
 // the thermally perfect instantiations exist for the FP64 form only
 template <class R>
 static void aux_launch(const Geom& g, DevState& d, int apply_shift, int write_ghost, int kid, cudaStream_t s,
-                       long long* nl, double* vel = nullptr) {
+                       long long* nl, double* vel = nullptr, bool dt = false) {
   if constexpr (sizeof(R) == sizeof(double)) {
     if (!g.calorically_perfect) {
-      aux_launch_tp<R, true>(g, d, apply_shift, write_ghost, kid, s, nl, vel);
+      aux_launch_tp<R, true>(g, d, apply_shift, write_ghost, kid, s, nl, vel, dt);
       return;
     }
   }
-  aux_launch_tp<R, false>(g, d, apply_shift, write_ghost, kid, s, nl, vel);
+  aux_launch_tp<R, false>(g, d, apply_shift, write_ghost, kid, s, nl, vel, dt);
 }
 
 cudaError_t launch_aux(const Geom& g, DevState& d, int apply_shift, cudaStream_t s, long long* nl) {
   if (g.precision == 1) aux_launch<float>(g, d, apply_shift, 0, K_AUX, s, nl);
   else aux_launch<double>(g, d, apply_shift, 0, K_AUX, s, nl);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_aux_dt(const Geom& g, DevState& d, int apply_shift, double cfl, cudaStream_t s, long long* nl) {
+  if (g.precision == 1) aux_launch<float>(g, d, apply_shift, 0, K_AUX, s, nl, nullptr, true);
+  else aux_launch<double>(g, d, apply_shift, 0, K_AUX, s, nl, nullptr, true);
+  SB_LAUNCH(d, K_DT_FINISH, s, k_dt_finish<<<1, FIN_NT, 0, s>>>(d.red, nblocks(g.nvol, AUX_NT), cfl, d.sc));
+  ++*nl;
   return cudaGetLastError();
 }
 
