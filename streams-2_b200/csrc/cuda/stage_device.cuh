@@ -39,8 +39,8 @@ constexpr int XF_TX = 32, XF_TY = 4, XF_NT = XF_TX * XF_TY;  // x faces: 4 row-w
 constexpr int MT_MAXW = 9, MT_SEG = 2048;
 // Registers of the flux kernels, as the threads an SM shall hold (y / z: 65536 / MT_MAXT_* registers
 // for blocks of any size) or the blocks of 128 (x, WENO faces).  The FP64 kernels want 128 registers
-// (1024x256x192 boundary layer, ms per step: y 12.2, z 13.6, x 11.5 at 16 warps per SM; at 20 warps
-// and 96 registers they spill 80-180 bytes: 13.2, 15.1, 12.1), the FP32 ones 80 (1024x256x128 shock
+// (1024x256x192 boundary layer, ms per step: y 11.5, z 13.2, x 11.0 at 16 warps per SM; at 20 warps
+// and 96 registers they spill 30-130 bytes: 12.7, 14.4, 11.8), the FP32 ones 80 (1024x256x128 shock
 // interaction: z 7.4, y 5.6 at 24 warps against 7.2, 5.7 at 20; 512x256x256 channel: z 5.9, y 3.1
 // against 6.1, 3.4; x 3.3 at 24 against 3.8 at 20).  The WENO face kernels' scattered stencils are
 // held in registers: 3 blocks (6.5 against 7.2 ms at 4) and 4 (1.9 against 2.1 ms at 5) in FP32.
@@ -563,9 +563,9 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group 
 // boundary layer, ms per step: 16.7 with the stencil loaded by every face into registers, 13.7 read
 // from L1 as often as used, 11.5 from the buffer.
 // fl is written (first contribution of the stage, euler_x after init_flux).
-// values of a thread's scratch (Scr): the two acoustic projections of the stencil's points
+// values of a thread's scratch (Scr): state and flux of the stencil's points on the two acoustic fields
 template <class R, int WS>
-constexpr int scr_vals() { return sizeof(R) == sizeof(double) ? 4 * WS : 0; }
+constexpr int scr_vals() { return sizeof(R) == sizeof(double) ? 8 * WS : 0; }
 constexpr int XG_MAX = 8, X_SMEM_MAX = 64 * 1024;
 struct XShape {
   int ngrp, slots;
@@ -717,9 +717,9 @@ __global__ void __launch_bounds__(XF_NT, sizeof(R) == 8 ? XF_MINB_D : XF_MINB_F)
 constexpr int MARCH_SMEM_MAX = 220 * 1024;
 __host__ __device__ __forceinline__ int ring_slots(int nw, int S) { return 2 * nw + 2 * S - 1; }
 template <class R, int LB, int WS>
-size_t march_smem(int nwarps, int seglen) {
+size_t march_smem(int nwarps, int seglen, bool split = false) {
   constexpr int S = LB > WS ? LB : WS;
-  return (size_t)(nwarps + 1) * 5 * 32 * 8 + (size_t)nwarps * 32 * scr_vals<R, WS>() * 8 +
+  return (size_t)(nwarps + 1) * 5 * 32 * 8 + (split ? 0 : (size_t)nwarps * 32 * scr_vals<R, WS>() * 8) +
          (size_t)ring_slots(nwarps, S) * ring_fields<R>() * 32 * sizeof(R) + ((size_t)seglen + 2 * WS) * 4;
 }
 template <class R, int DIR, int LB, int WS, bool CH = false, int FS = 0, bool SPLIT = false>
@@ -738,7 +738,7 @@ __device__ __forceinline__ void d_march(const Geom& g, const R* __restrict__ aux
   const int nslot = ring_slots(nw, S);
   double* scd = xch + (nw + 1) * 5 * 32;
   const Scr<R> scr{(unsigned)__cvta_generic_to_shared(scd + threadIdx.x), blockDim.x * 8};
-  R* ring = reinterpret_cast<R*>(scd + scr_vals<R, WS>() * blockDim.x);
+  R* ring = reinterpret_cast<R*>(scd + (SPLIT ? 0 : scr_vals<R, WS>() * blockDim.x));  // no WENO face is computed in the split form
   unsigned* flag = reinterpret_cast<unsigned*>(ring + nslot * RF * 32);
   const unsigned ring_a = (unsigned)__cvta_generic_to_shared(ring) + lane * (unsigned)sizeof(R);
   const int n1 = g.nx;

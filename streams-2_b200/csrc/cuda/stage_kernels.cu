@@ -174,6 +174,7 @@ static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, do
   if (a.run_aux) aux_launch<R>(g, d, a.apply_shift, 0, K_AUX, s, nl, vel);
   const size_t ysm = march_smem<R, LB, WS>(my.nwarps, my.seglen);
   const size_t zsm = march_smem<R, LB, WS>(mz.nwarps, mz.seglen);
+  const size_t yss = march_smem<R, LB, WS>(my.nwarps, my.seglen, true), zss = march_smem<R, LB, WS>(mz.nwarps, mz.seglen, true);
   // per instantiation and device: allow more than 48 KB of dynamic shared memory
   static unsigned long long smem_set = 0;
   int dev = 0;
@@ -254,7 +255,7 @@ static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, do
                                                           a.rhork, a.gamrk, a.istep, my.seglen, my.nseg, d.red));
     if (split_on) {
       SB_LAUNCH(d, K_EULER_Y, s,
-                k_march<R, 1, LB, WS, false, FS, true><<<my.nblk, 32 * my.nwarps, ysm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
+                k_march<R, 1, LB, WS, false, FS, true><<<my.nblk, 32 * my.nwarps, yss, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
                                                                    d.sc, a.rhork, a.gamrk, a.istep, my.seglen, my.nseg, d.red));
       ++*nl;
     }
@@ -270,7 +271,7 @@ static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, do
                                                                   a.rhork, a.gamrk, a.istep, mz.seglen, mz.nseg, d.red));
     if (split_on)
       SB_LAUNCH(d, K_EULER_Z, s,
-                k_march<R, 2, LB, WS, true, FS, true><<<mz.nblk, 32 * mz.nwarps, zsm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
+                k_march<R, 2, LB, WS, true, FS, true><<<mz.nblk, 32 * mz.nwarps, zss, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
                                                                   d.sc, a.rhork, a.gamrk, a.istep, mz.seglen, mz.nseg, d.red));
   } else {
     SB_LAUNCH(d, K_EULER_Z, s,
@@ -278,7 +279,7 @@ static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, do
                                                                    a.rhork, a.gamrk, a.istep, mz.seglen, mz.nseg, d.red));
     if (split_on)
       SB_LAUNCH(d, K_EULER_Z, s,
-                k_march<R, 2, LB, WS, false, FS, true><<<mz.nblk, 32 * mz.nwarps, zsm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
+                k_march<R, 2, LB, WS, false, FS, true><<<mz.nblk, 32 * mz.nwarps, zss, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
                                                                    d.sc, a.rhork, a.gamrk, a.istep, mz.seglen, mz.nseg, d.red));
   }
   if (split_on) ++*nl;
