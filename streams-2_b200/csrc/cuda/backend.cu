@@ -244,17 +244,9 @@ void fill_geom(streams_b200_ctx* c) {
     g.weps_a = 0.000001 * r2u2;
     g.weps_b = 0.000001 * r2u4;
     g.weps_c = 0.000001 * r2u6;
-    auto pow2 = [](double v) { return std::exp2(std::round(std::log2(v > 0.0 && std::isfinite(v) ? v : 1.0))); };
-    g.wsg_a = pow2(1.0 / std::sqrt(r2u2));
-    g.wsg_b = pow2(1.0 / std::sqrt(r2u4));
-    g.wsg_c = pow2(1.0 / std::sqrt(r2u6));
-    g.wsg_ai = 1.0 / g.wsg_a;
-    g.wsg_bi = 1.0 / g.wsg_b;
-    g.wsg_ci = 1.0 / g.wsg_c;
-    g.wepsf_a = g.weps_a * g.wsg_a * g.wsg_a;
-    g.wepsf_b = g.weps_b * g.wsg_b * g.wsg_b;
-    g.wepsf_c = g.weps_c * g.wsg_c * g.wsg_c;
-    g.wepsf_ab = g.weps_b * g.wsg_a * g.wsg_a;
+    g.wbs_a = 1.0 / r2u2;
+    g.wbs_b = 1.0 / r2u4;
+    g.wbs_c = g.wbs_b / u0_2;
   }
   g.calorically_perfect = p.calorically_perfect;
   g.cp_l = p.indx_cp_l;
@@ -405,20 +397,24 @@ int streams_b200_create(const streams_b200_params* p, const streams_b200_grid* g
       g.vrl[d] = dr - 1;
       g.vhl[d] = dh - 1;
       g.vrlf[d] = drf - 1;
-      std::vector<double> fr(nn[d] + 1);
-      std::vector<float> frf(nn[d] + 1);
-      for (int i = 0; i <= nn[d]; ++i) {
-        fr[i] = 1.0 / (crd[d][i + ng] - crd[d][i + ng - 1]);
-        frf[i] = static_cast<float>(fr[i]);
+      const int nf = nn[d] + 1;
+      std::vector<double> fr(nf);
+      std::vector<float> ff(2 * nf);
+      for (int i = 0; i < nf; ++i) {
+        const double dd = crd[d][i + ng] - crd[d][i + ng - 1];  // x(i+1) - x(i)
+        fr[i] = 1.0 / dd;
+        ff[i] = static_cast<float>(dd);
+        ff[nf + i] = 1.0f / ff[i];
       }
       double* df;
       float* dff;
-      if ((e = dev_alloc(c, &df, nn[d] + 1)) || (e = dev_alloc(c, &dff, nn[d] + 1))) return fail(e, "cudaMalloc(grid)");
-      if ((e = cudaMemcpy(df, fr.data(), (nn[d] + 1) * 8, cudaMemcpyHostToDevice)) ||
-          (e = cudaMemcpy(dff, frf.data(), (nn[d] + 1) * 4, cudaMemcpyHostToDevice)))
+      if ((e = dev_alloc(c, &df, nf)) || (e = dev_alloc(c, &dff, 2 * nf))) return fail(e, "cudaMalloc(grid)");
+      if ((e = cudaMemcpy(df, fr.data(), nf * 8, cudaMemcpyHostToDevice)) ||
+          (e = cudaMemcpy(dff, ff.data(), 2 * nf * 4, cudaMemcpyHostToDevice)))
         return fail(e, "cudaMemcpy(grid)");
       g.vfr[d] = df;
-      g.vfrf[d] = dff;
+      g.vfdf[d] = dff;
+      g.vfrf[d] = dff + nf;
     }
   }
   g.yn = dyn - 1;

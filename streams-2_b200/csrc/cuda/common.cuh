@@ -33,8 +33,9 @@ struct Geom {
   const double* vrl[3];
   const float* vrlf[3];
   const double* vhl[3];
-  // 1/(x(i+1)-x(i)) of the faces i = 0..n
+  // of the faces i = 0..n, 1/(x(i+1)-x(i)) in FP64, and x(i+1)-x(i) and its reciprocal in FP32
   const double* vfr[3];
+  const float* vfdf[3];
   const float* vfrf[3];
   const double* y;
   const double* z;
@@ -82,14 +83,11 @@ struct Geom {
   int visc_model;
   double mu0, t0, rgas0, rho0, u0, l0, sutherland_s, t_ref_dim, vtexp, prandtl;
   double cp0, cv0, cp_last, cv_last, gamloc;
-  // constants of the WENO faces formed once on the host: gamma - 1, 1/(gamma - 1) and 1/cp of the
-  // calorically perfect gas, and the 1e-6 of the weights over the smoothness-indicator scales
-  // 1/(rho0^2 u0^2) and 1/(rho0^2 u0^4) of wenorec_1d (kernels_cpu.F90:2539-2546) and
-  // 1/(rho0^2 u0^6).  FP32 values are scaled by powers of two wsg near the square roots of those
-  // scales (wsg_*i their reciprocals): wepsf = wsg^2 weps, wepsf_ab with the scale b and wsg_a
-  double gm1, rgm1, rcp0, rcv0, rt0, cpp, rpr;  // 1/cp, 1/cv, 1/t0, cp/Pr, 1/Pr
-  double weps_a, weps_b, weps_c;
-  double wsg_a, wsg_b, wsg_c, wsg_ai, wsg_bi, wsg_ci, wepsf_a, wepsf_b, wepsf_c, wepsf_ab;
+  // constants formed once on the host: gamma - 1, 1/(gamma - 1) of the calorically perfect gas, 1/cp,
+  // 1/cv, 1/t0, cp/Pr and 1/Pr, the smoothness-indicator scales 1/(rho0^2 u0^2) and
+  // 1/(rho0^2 u0^4) of wenorec_1d (kernels_cpu.F90:2539-2546) and 1/(rho0^2 u0^6), and its 1e-6 over
+  // each of them
+  double gm1, rgm1, rcp0, rcv0, rt0, cpp, rpr, wbs_a, wbs_b, wbs_c, weps_a, weps_b, weps_c;
   // thermally perfect gas (calorically_perfect = 0): cp(T) = sum of cpc[l - cp_l] (T/t0)^l for
   // l = cp_l..cp_r, cv likewise (set_fluid_prop's cp_coeff / cv_coeff, times rgas0)
   int calorically_perfect, cp_l, cp_r;

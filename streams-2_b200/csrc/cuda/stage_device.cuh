@@ -4,11 +4,11 @@
 //   k_apply_shift  the pending force_var energy shift of the previous stage, on interior w
 //   k_aux      w -> primitive/thermo fields at interior and face-ghost points; ghost values are
 //              produced on the fly (periodic wrap, staggered isothermal wall mirror)
-//   k_xflux    x-face hybrid fluxes + divergence (fl = ...); a warp holds 32 consecutive faces of
-//              the rows' face sequence, shuffles between lanes
-//   k_visc     reduced 2nd-order viscous terms, conservative face Laplacian in x, y, z,
-//              div/3, stage-3 Ducros sensor, wall shear
-//   k_march<1> y-face fluxes + divergence (fl += ...); register-window march along y lines
+//   k_xflux    x-face hybrid fluxes + divergence (fl = ...); a warp takes groups of 32 consecutive
+//              faces of the rows' face sequence from a buffer of its own, shuffles between lanes
+//   k_visc_tiled  reduced 2nd-order viscous terms, conservative face Laplacian in x, y, z,
+//              div/3, stage-3 Ducros sensor, wall shear; planes in a ring in shared memory
+//   k_march<1> y-face fluxes + divergence (fl += ...); rounds of faces from a ring in shared memory
 //   k_march<2> z-face fluxes + divergence + grad(mu div/3) term; block partials of force_rhs
 //   k_finish_rhs  bulk quantities and the forcing correction (deterministic order)
 //   k_update   RK register fln, forcing correction, w += fln, force_var / residual partials
@@ -19,12 +19,13 @@
 // Precision: template parameter R is the arithmetic type of the fluxes and viscous terms and the
 // storage type of the primitive fields (aux) and div/3.  R = double is the FP64 form; R = float
 // the mixed form, where w, the RK registers fl, the temperature recovery from the total energy,
-// the Ducros sensor, the time step and all reductions stay FP64 and the face fluxes are carried
-// as float-float pairs whose differences are formed in FP64.
+// the Ducros sensor, the time step and all reductions stay FP64 and the face fluxes are summed and
+// differenced in FP64.
 #pragma once
 
 #include <algorithm>
 #include <cfloat>
+#include <type_traits>
 
 #include "flux.cuh"
 #include "kernels.hpp"
@@ -38,17 +39,18 @@ constexpr int XF_TX = 32, XF_TY = 4, XF_NT = XF_TX * XF_TY;  // x faces: 4 row-w
 // y / z passes: blocks of LW = 4 warps, up to MT_MAXW in small boxes; segments of at most MT_SEG cells
 constexpr int MT_MAXW = 9, MT_SEG = 2048;
 // Registers of the flux kernels, as the threads an SM shall hold (y / z: 65536 / MT_MAXT_* registers
-// for blocks of any size) or the blocks of 128 (x, WENO faces).  The FP64 kernels want 128 registers
-// (1024x256x192 boundary layer, ms per step: y 11.5, z 13.2, x 11.0 at 16 warps per SM; at 20 warps
-// and 96 registers they spill 30-130 bytes: 12.7, 14.4, 11.8), the FP32 ones 80 (1024x256x128 shock
-// interaction: z 7.4, y 5.6 at 24 warps against 7.2, 5.7 at 20; 512x256x256 channel: z 5.9, y 3.1
-// against 6.1, 3.4; x 3.3 at 24 against 3.8 at 20).  The WENO face kernels' scattered stencils are
-// held in registers: 3 blocks (6.5 against 7.2 ms at 4) and 4 (1.9 against 2.1 ms at 5) in FP32.
+// for blocks of any size) or the blocks of 128 (x, WENO faces).  FP64 takes 128 registers
+// (1024x256x192 boundary layer, ms per step: y 11.0, z 12.5, x 10.7 at 16 warps per SM, without
+// spills; an earlier form at 20 warps and 96 registers, spilling 30-130 bytes: 12.7, 14.4, 11.8
+// against 11.5, 13.2, 11.0).  FP32: 96 in y and z (1024x256x128 shock interaction z 8.7, y 7.2
+// against 9.3, 7.3 at 80; 512x256x256 channel 5.8, 3.3 against 5.8, 3.1), 80 in x (6.9 and 2.8
+// against 7.1 and 2.9 at 96).  The WENO face kernels' scattered stencils: 3 blocks (6.5 against
+// 7.2 ms at 4) and 4 in FP32.
 #ifndef MT_MAXT_D
 #define MT_MAXT_D 512
 #endif
 #ifndef MT_MAXT_F
-#define MT_MAXT_F 768
+#define MT_MAXT_F 640
 #endif
 #ifndef XF_MINB_D
 #define XF_MINB_D 4
@@ -440,11 +442,23 @@ __device__ __forceinline__ R line_r(const Geom& g, int d, int i) {
   else return __ldg(g.vrlf[d] + i);
 }
 
-// 1/(x(i+1)-x(i)) likewise, i = 0 .. n
+// Quotient by a value b that comes with its rounded reciprocal r: a product in FP64; in FP32 the
+// rounded quotient itself (a r corrected by its remainder, Markstein), so that the mixed form's FP32
+// results are those of a division.
 template <class R>
-__device__ __forceinline__ R face_r(const Geom& g, int d, int i) {
-  if constexpr (sizeof(R) == sizeof(double)) return __ldg(g.vfr[d] + i);
-  else return __ldg(g.vfrf[d] + i);
+struct Quot {
+  R b, r;
+};
+__device__ __forceinline__ double quot(double a, const Quot<double>& q) { return a * q.r; }
+__device__ __forceinline__ float quot(float a, const Quot<float>& q) {
+  const float t = __fmul_rn(a, q.r);
+  return __fmaf_rn(q.r, __fmaf_rn(-q.b, t, a), t);
+}
+// x(i+1)-x(i) of a face and its reciprocal, i = 0 .. n
+template <class R>
+__device__ __forceinline__ Quot<R> face_r(const Geom& g, int d, int i) {
+  if constexpr (sizeof(R) == sizeof(double)) return Quot<R>{R(0), __ldg(g.vfr[d] + i)};
+  else return Quot<R>{__ldg(g.vfdf[d] + i), __ldg(g.vfrf[d] + i)};
 }
 
 template <int DIR>
@@ -518,10 +532,14 @@ __host__ __device__ __forceinline__ long long wface_count(const Geom& g) {
 template <class R, int DIR, int LB, int WS, int S, int FS, class LN>
 __device__ __forceinline__ void weno_face(const Geom& g, const LN& ln, int ep, double (&f)[5], const Scr<R>& scr) {
   const int ord = max(WS + ep, 1);
-  if constexpr ((FS & 1) != 0)
-    rusanov_flux<R, DIR, WS, S, (FS & 2) != 0, (FS & 8) != 0>(g, ln, ord, f);
-  else
-    weno_flux<R, DIR, WS, S, (FS & 2) != 0, (FS & 8) != 0>(g, ln, ord, f, scr);
+  auto flux = [&](auto full) {
+    constexpr bool FULL = decltype(full)::value;
+    if constexpr ((FS & 1) != 0) rusanov_flux<R, DIR, WS, S, (FS & 2) != 0, (FS & 8) != 0, FULL>(g, ln, ord, f);
+    else if constexpr (sizeof(R) == sizeof(double)) weno_flux<DIR, WS, S, (FS & 2) != 0, (FS & 8) != 0, FULL>(g, ln, ord, f, scr);
+    else weno_flux_f<DIR, WS, S, (FS & 8) != 0>(g, ln, ord, f, scr);
+  };
+  if (sizeof(R) != sizeof(double) || ord == WS) flux(std::true_type{});
+  else flux(std::false_type{});
 }
 
 template <class R, int DIR, int LB, int WS, int S, int FS, class LN>
@@ -563,9 +581,6 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group 
 // boundary layer, ms per step: 16.7 with the stencil loaded by every face into registers, 13.7 read
 // from L1 as often as used, 11.5 from the buffer.
 // fl is written (first contribution of the stage, euler_x after init_flux).
-// values of a thread's scratch (Scr): state and flux of the stencil's points on the two acoustic fields
-template <class R, int WS>
-constexpr int scr_vals() { return sizeof(R) == sizeof(double) ? 8 * WS : 0; }
 constexpr int XG_MAX = 8, X_SMEM_MAX = 64 * 1024;
 struct XShape {
   int ngrp, slots;
@@ -574,7 +589,7 @@ struct XShape {
 __host__ __device__ __forceinline__ int x_slots(int nx, int S) { return 32 + (2 * S - 1) * ((31 + nx) / (nx + 1) + 1); }
 template <class R, int WS>
 __host__ __device__ __forceinline__ size_t x_warp_bytes(int slots) {
-  return 2 * (size_t)((slots * XS * (int)sizeof(R) + 7) / 8 * 8 + slots * 8) + 5 * 8 + scr_vals<R, WS>() * 32 * 8;
+  return 2 * (size_t)((slots * XS * (int)sizeof(R) + 7) / 8 * 8 + slots * 8) + 5 * 8 + scr_vals<R, WS>() * 32 * sizeof(R);
 }
 template <class R, int LB, int WS, int FS = 0>
 __device__ __forceinline__ void d_xflux(const Geom& g, const R* __restrict__ aux, const double* __restrict__ sensor,
@@ -587,8 +602,8 @@ __device__ __forceinline__ void d_xflux(const Geom& g, const R* __restrict__ aux
   if (fw0 >= nface) return;  // whole warp leaves together
   const unsigned nmine = (unsigned)min((unsigned long long)(32 * ngrp), nface - fw0);  // this warp's faces
   unsigned char* wm = sb_dyn_smem + threadIdx.y * x_warp_bytes<R, WS>(slots);
-  const Scr<R> scr{(unsigned)__cvta_generic_to_shared(wm) + lane * 8, 32 * 8};
-  wm += scr_vals<R, WS>() * 32 * 8;
+  const Scr<R> scr{reinterpret_cast<R*>(wm) + lane, 32};
+  wm += scr_vals<R, WS>() * 32 * sizeof(R);
   double* carry = reinterpret_cast<double*>(wm);  // the group before's last face
   const unsigned pb = (unsigned)((slots * XS * (int)sizeof(R) + 7) / 8 * 8);  // bytes of a buffer's points
   unsigned char* buf0 = wm + 5 * 8;
@@ -607,11 +622,14 @@ __device__ __forceinline__ void d_xflux(const Geom& g, const R* __restrict__ aux
     }
     return q;
   };
+  // rows between the row of a group's first face and that of the face n after the row's face 0 (a
+  // group touches two rows at most unless the rows are shorter than a warp)
+  auto rows_on = [&](int n) { return n < nfr ? 0 : (n < 2 * nfr ? 1 : n / nfr); };
   auto fetch = [&](const Pos& q0, int nf, int bi) {  // the points of the nf faces from q0 on
     unsigned char* pts = buf0 + bi * (pb + slots * 8);
     double* sen = reinterpret_cast<double*>(pts + pb);
     const int n0 = nfr - q0.p;  // faces left in the first row
-    const int total = nf + W2 * ((q0.p + nf - 1) / nfr + 1);
+    const int total = nf + W2 * (rows_on(q0.p + nf - 1) + 1);
     for (int s = lane; s < total; s += 32) {
       Pos q = q0;
       int t = s;
@@ -651,7 +669,7 @@ __device__ __forceinline__ void d_xflux(const Geom& g, const R* __restrict__ aux
     const Pos qn = forward(q0, 32);
     // this lane's face (between the points p and p+1) and its first stencil point
     const Pos q = forward(q0, lane);
-    const int s0 = lane + W2 * ((q0.p + lane) / nfr);
+    const int s0 = lane + W2 * rows_on(q0.p + lane);
     const int p = q.p;
     const bool in = lane < nf;
     const int ep = in ? face_ep<0>(g, p) : 0;
@@ -719,7 +737,7 @@ __host__ __device__ __forceinline__ int ring_slots(int nw, int S) { return 2 * n
 template <class R, int LB, int WS>
 size_t march_smem(int nwarps, int seglen, bool split = false) {
   constexpr int S = LB > WS ? LB : WS;
-  return (size_t)(nwarps + 1) * 5 * 32 * 8 + (split ? 0 : (size_t)nwarps * 32 * scr_vals<R, WS>() * 8) +
+  return (size_t)(nwarps + 1) * 5 * 32 * 8 + (split ? 0 : (size_t)nwarps * 32 * scr_vals<R, WS>() * sizeof(R)) +
          (size_t)ring_slots(nwarps, S) * ring_fields<R>() * 32 * sizeof(R) + ((size_t)seglen + 2 * WS) * 4;
 }
 template <class R, int DIR, int LB, int WS, bool CH = false, int FS = 0, bool SPLIT = false>
@@ -736,9 +754,9 @@ __device__ __forceinline__ void d_march(const Geom& g, const R* __restrict__ aux
   double* xch = reinterpret_cast<double*>(sb_dyn_smem);
   constexpr int RF = ring_fields<R>();
   const int nslot = ring_slots(nw, S);
-  double* scd = xch + (nw + 1) * 5 * 32;
-  const Scr<R> scr{(unsigned)__cvta_generic_to_shared(scd + threadIdx.x), blockDim.x * 8};
-  R* ring = reinterpret_cast<R*>(scd + (SPLIT ? 0 : scr_vals<R, WS>() * blockDim.x));  // no WENO face is computed in the split form
+  R* scd = reinterpret_cast<R*>(xch + (nw + 1) * 5 * 32);
+  const Scr<R> scr{scd + threadIdx.x, (int)blockDim.x};
+  R* ring = (scd + (SPLIT ? 0 : scr_vals<R, WS>() * blockDim.x));  // no WENO face is computed in the split form
   unsigned* flag = reinterpret_cast<unsigned*>(ring + nslot * RF * 32);
   const unsigned ring_a = (unsigned)__cvta_generic_to_shared(ring) + lane * (unsigned)sizeof(R);
   const int n1 = g.nx;
@@ -861,8 +879,15 @@ __device__ __forceinline__ void d_march(const Geom& g, const R* __restrict__ aux
         const int j = b, k = c;
         R sigx, sigy, sigz;
         if (g.conservative_viscous) {
-          // mu times the per-line 1/(x(i+1)-x(i-1))
-          const R dxl = mu * line_r<R>(g, 0, i), dyl = mu * line_r<R>(g, 1, j), dzl = mu * line_r<R>(g, 2, k);
+          // mu/(x(i+1)-x(i-1)): in FP64 by the per-line reciprocals, in FP32 the rounded quotient
+          R dxl, dyl, dzl;
+          if constexpr (sizeof(R) == sizeof(double)) {
+            dxl = mu * line_r<R>(g, 0, i); dyl = mu * line_r<R>(g, 1, j); dzl = mu * line_r<R>(g, 2, k);
+          } else {
+            dxl = mu / R(g.x[i + 1] - g.x[i - 1]);
+            dyl = mu / R(g.y[j + 1] - g.y[j - 1]);
+            dzl = mu / R(g.z[k + 1] - g.z[k - 1]);
+          }
           sigx = dxl * (dv[0] - dv[1]);
           sigy = dyl * (dv[2] - dv[3]);
           sigz = dzl * (dv[4] - dv[5]);
@@ -1017,7 +1042,7 @@ __device__ __forceinline__ void d_visc_tiled(const Geom& g, const R* __restrict_
   load_plane(k0 + 1);
   load_fl(k0);
   copy_commit();
-  const R cpp = TP ? R(0) : R(g.cpp), rpr = R(g.rpr);
+  const R cpp = R(g.cpp), rpr = sizeof(R) == sizeof(double) ? R(g.rpr) : R(1) / R(g.prandtl);
   R zlo[4] = {R(0), R(0), R(0), R(0)};  // flux of the lower z face
   for (int k = k0; k <= k1; ++k) {
     copy_wait<0>();
@@ -1040,39 +1065,42 @@ __device__ __forceinline__ void d_visc_tiled(const Geom& g, const R* __restrict_
       const R qc = R(0.5) * (c0[0] * c0[0] + c0[1] * c0[1] + c0[2] * c0[2]);
       // conservative face Laplacian: flux at the face between the cell and its neighbour o of plane
       // p at distance 1/rd, for the cell below (sgn = 1) or above (-1) the face
-      auto face = [&](const R* p, int o, R rd, R sgn, R (&s)[4]) {
+      auto face = [&](const R* p, int o, const Quot<R>& rd, R sgn, R (&s)[4]) {
         const R u = F(p, o, 0), v = F(p, o, 1), w = F(p, o, 2), t = F(p, o, 3);
-        const R muf = (R(0.5) * (F(p, o, 4) + c0[4])) * (rd * sgn);
+        const R muf = quot(R(0.5) * (F(p, o, 4) + c0[4]), rd) * sgn;
         const R qn = R(0.5) * (u * u + v * v + w * w);
         s[0] = (u - c0[0]) * muf;
         s[1] = (v - c0[1]) * muf;
         s[2] = (w - c0[2]) * muf;
-        const R cpf = TP ? R(cp_of_t(g, double(R(0.5) * (t + c0[3])))) * rpr : cpp;
-        s[3] = ((t - c0[3]) * cpf + (qn - qc)) * muf;
+        R heat;  // (T - T0) cp/Pr
+        if constexpr (TP) heat = (t - c0[3]) * (R(cp_of_t(g, double(R(0.5) * (t + c0[3])))) * rpr);
+        else if constexpr (sizeof(R) == sizeof(double)) heat = (t - c0[3]) * cpp;
+        else heat = quot((t - c0[3]) * R(g.cp0), Quot<R>{R(g.prandtl), rpr});
+        s[3] = (heat + (qn - qc)) * muf;
       };
       R lo[4], hi[4];
       // x: fl += dxhl*(fhat(i) - fhat(i-1)), fhat = -sigma
       face(p0, -1, face_r<R>(g, 0, i - 1), R(-1), lo);
       face(p0, 1, face_r<R>(g, 0, i), R(1), hi);
       const double dxhl = __ldg(g.vhl[0] + i);
-      f2 = f2 + dxhl * double(lo[0] - hi[0]);
-      f3 = f3 + dxhl * double(lo[1] - hi[1]);
-      f4 = f4 + dxhl * double(lo[2] - hi[2]);
-      f5 = f5 + dxhl * double(lo[3] - hi[3]);
+      f2 = f2 + dxhl * (double(lo[0]) - double(hi[0]));
+      f3 = f3 + dxhl * (double(lo[1]) - double(hi[1]));
+      f4 = f4 + dxhl * (double(lo[2]) - double(hi[2]));
+      f5 = f5 + dxhl * (double(lo[3]) - double(hi[3]));
       face(p0, -VT_PX, face_r<R>(g, 1, j - 1), R(-1), lo);
       face(p0, VT_PX, face_r<R>(g, 1, j), R(1), hi);
       const double dyhl = __ldg(g.vhl[1] + j);
-      f2 = f2 + dyhl * double(lo[0] - hi[0]);
-      f3 = f3 + dyhl * double(lo[1] - hi[1]);
-      f4 = f4 + dyhl * double(lo[2] - hi[2]);
-      f5 = f5 + dyhl * double(lo[3] - hi[3]);
+      f2 = f2 + dyhl * (double(lo[0]) - double(hi[0]));
+      f3 = f3 + dyhl * (double(lo[1]) - double(hi[1]));
+      f4 = f4 + dyhl * (double(lo[2]) - double(hi[2]));
+      f5 = f5 + dyhl * (double(lo[3]) - double(hi[3]));
       if (k == k0) face(pm, 0, face_r<R>(g, 2, k - 1), R(-1), zlo);
       face(pp, 0, face_r<R>(g, 2, k), R(1), hi);
       const double dzhl = __ldg(g.vhl[2] + k);
-      f2 = f2 + dzhl * double(zlo[0] - hi[0]);
-      f3 = f3 + dzhl * double(zlo[1] - hi[1]);
-      f4 = f4 + dzhl * double(zlo[2] - hi[2]);
-      f5 = f5 + dzhl * double(zlo[3] - hi[3]);
+      f2 = f2 + dzhl * (double(zlo[0]) - double(hi[0]));
+      f3 = f3 + dzhl * (double(zlo[1]) - double(hi[1]));
+      f4 = f4 + dzhl * (double(zlo[2]) - double(hi[2]));
+      f5 = f5 + dzhl * (double(zlo[3]) - double(hi[3]));
 #pragma unroll
       for (int m = 0; m < 4; ++m) zlo[m] = hi[m];
       // reduced second-order terms
@@ -1097,7 +1125,10 @@ __device__ __forceinline__ void d_visc_tiled(const Geom& g, const R* __restrict_
         wallprop[nw + wp] = double(c0[4] * wy);
         wallprop[2 * nw + wp] = double(c0[4] * ty_ * cploc / R(g.prandtl));
       }
-      const R div3l = (ux + vy + wz) * R(1.0 / 3.0);
+      R div;  // with the rounding of the mixed form fixed: du/dx fused with the first sum only
+      if constexpr (sizeof(R) == sizeof(double)) div = ux + vy + wz;
+      else div = __fadd_rn(__fmaf_rn(dxl, F(p0, 1, 0) - F(p0, -1, 0), vy), wz);
+      const R div3l = quot(div, Quot<R>{R(3), R(1.0 / 3.0)});
       div3[q] = div3l;
       if (do_sensor) {
         // sensor_subroutine works from the stored |omega| and div/3
@@ -1109,12 +1140,14 @@ __device__ __forceinline__ void d_visc_tiled(const Geom& g, const R* __restrict_
         const R t = fmax(-dv / sqrt(om2 + dv * dv + u0l0 * u0l0), R(0));
         sensor_next[q] = double(t * t);
       }
-      const R d2 = R(2) * div3l;
-      const R sig11 = ux - d2, sig22 = vy - d2, sig33 = wz - d2;
-      const R sigx = mux * sig11 + muy * vx + muz * wx;
-      const R sigy = mux * uy + muy * sig22 + muz * wy;
-      const R sigz = mux * uz + muy * vz + muz * sig33;
-      const R sigah = (sig11 * ux + sig22 * vy + sig33 * wz + R(2) * (vx * uy + wx * uz + wy * vz)) * c0[4];
+      const R sig11 = ux - R(2) * div3l, sig12 = vx, sig13 = wx;
+      const R sig21 = uy, sig22 = vy - R(2) * div3l, sig23 = wy;
+      const R sig31 = uz, sig32 = vz, sig33 = wz - R(2) * div3l;
+      const R sigx = mux * sig11 + muy * sig12 + muz * sig13;
+      const R sigy = mux * sig21 + muy * sig22 + muz * sig23;
+      const R sigz = mux * sig31 + muy * sig32 + muz * sig33;
+      const R sigah = (sig11 * ux + sig12 * uy + sig13 * uz + sig21 * vx + sig22 * vy + sig23 * vz + sig31 * wx +
+                       sig32 * wy + sig33 * wz) * c0[4];
       const R sigq = sigx * c0[0] + sigy * c0[1] + sigz * c0[2] + sigah;
       fl[nI + q] = f2 - double(sigx);
       fl[2 * nI + q] = f3 - double(sigy);
@@ -1695,11 +1728,8 @@ __global__ void __launch_bounds__(WF_NT, sizeof(R) == 8 ? WF_MINB_D : WF_MINB_F)
     const long long base = DIR == 0 ? gidx(g, p, a, b) : (DIR == 1 ? gidx(g, a, p, b) : gidx(g, a, b, p));
     const Line<R> ln{aux + base - (S - 1) * sd, n, sd};
     double fw[5];
-    Scr<R> scr{0, 0};
-    if constexpr (scr_vals<R, WS>() > 0) {
-      __shared__ double wsc[scr_vals<R, WS>() * WF_NT];
-      scr = Scr<R>{(unsigned)__cvta_generic_to_shared(wsc + threadIdx.x), WF_NT * 8};
-    }
+    __shared__ R wsc[scr_vals<R, WS>() * WF_NT];
+    const Scr<R> scr{wsc + threadIdx.x, WF_NT};
     weno_face<R, DIR, LB, WS, S, FS>(g, ln, face_ep<DIR>(g, p), fw, scr);
 #pragma unroll
     for (int m = 0; m < 5; ++m) g.wface[m * g.nwface + f] = fw[m];
