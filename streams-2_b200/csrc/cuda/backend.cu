@@ -378,43 +378,33 @@ int streams_b200_create(const streams_b200_params* p, const streams_b200_grid* g
     const double* crd[3] = {gr->x, gr->y, gr->z};
     const int nn[3] = {p->nx, p->ny, p->nz};
     for (int d = 0; d < 3; ++d) {
-      std::vector<double> r(nn[d]), h(nn[d]);
-      std::vector<float> rf(nn[d]);
-      for (int i = 1; i <= nn[d]; ++i) {
+      // one buffer per direction: n, n and nf values in FP64, then n, nf and nf in FP32
+      const int n = nn[d], nf = n + 1;
+      std::vector<double> buf(2 * n + nf + (n + 2 * nf + 1) / 2);
+      double *r = buf.data(), *h = r + n, *fr = h + n;
+      float *rf = reinterpret_cast<float*>(fr + nf), *fd = rf + n, *frf = fd + nf;
+      for (int i = 1; i <= n; ++i) {
         const double dd = crd[d][i + ng] - crd[d][i + ng - 2];  // x(i+1) - x(i-1)
         r[i - 1] = 1.0 / dd;
         h[i - 1] = 2.0 / dd;
         rf[i - 1] = 1.0f / static_cast<float>(dd);
       }
-      double *dr, *dh;
-      float* drf;
-      if ((e = dev_alloc(c, &dr, nn[d])) || (e = dev_alloc(c, &dh, nn[d])) || (e = dev_alloc(c, &drf, nn[d])))
-        return fail(e, "cudaMalloc(grid)");
-      if ((e = cudaMemcpy(dr, r.data(), nn[d] * 8, cudaMemcpyHostToDevice)) ||
-          (e = cudaMemcpy(dh, h.data(), nn[d] * 8, cudaMemcpyHostToDevice)) ||
-          (e = cudaMemcpy(drf, rf.data(), nn[d] * 4, cudaMemcpyHostToDevice)))
-        return fail(e, "cudaMemcpy(grid)");
-      g.vrl[d] = dr - 1;
-      g.vhl[d] = dh - 1;
-      g.vrlf[d] = drf - 1;
-      const int nf = nn[d] + 1;
-      std::vector<double> fr(nf);
-      std::vector<float> ff(2 * nf);
       for (int i = 0; i < nf; ++i) {
         const double dd = crd[d][i + ng] - crd[d][i + ng - 1];  // x(i+1) - x(i)
         fr[i] = 1.0 / dd;
-        ff[i] = static_cast<float>(dd);
-        ff[nf + i] = 1.0f / ff[i];
+        fd[i] = static_cast<float>(dd);
+        frf[i] = 1.0f / fd[i];
       }
-      double* df;
-      float* dff;
-      if ((e = dev_alloc(c, &df, nf)) || (e = dev_alloc(c, &dff, 2 * nf))) return fail(e, "cudaMalloc(grid)");
-      if ((e = cudaMemcpy(df, fr.data(), nf * 8, cudaMemcpyHostToDevice)) ||
-          (e = cudaMemcpy(dff, ff.data(), 2 * nf * 4, cudaMemcpyHostToDevice)))
-        return fail(e, "cudaMemcpy(grid)");
-      g.vfr[d] = df;
-      g.vfdf[d] = dff;
-      g.vfrf[d] = dff + nf;
+      double* t;
+      if ((e = dev_alloc(c, &t, buf.size()))) return fail(e, "cudaMalloc(grid)");
+      if ((e = cudaMemcpy(t, buf.data(), buf.size() * 8, cudaMemcpyHostToDevice))) return fail(e, "cudaMemcpy(grid)");
+      float* tf = reinterpret_cast<float*>(t + 2 * n + nf);
+      g.vrl[d] = t - 1;
+      g.vhl[d] = t + n - 1;
+      g.vfr[d] = t + 2 * n;
+      g.vrlf[d] = tf - 1;
+      g.vfdf[d] = tf + n;
+      g.vfrf[d] = tf + n + nf;
     }
   }
   g.yn = dyn - 1;

@@ -162,13 +162,12 @@ __global__ void __launch_bounds__(FIN_NT) kb_finish_rhs(const BoxRec* __restrict
   d_finish_rhs(gs, r->red, r->nb_z, first_stage, r->sc, Blk{0, 0, 0});
 }
 
-template <unsigned SPAN, class R, bool TP>
+template <unsigned SPAN, class R, bool TP, int MODE>
 __global__ void __launch_bounds__(UPD_NT, UPD_MINB) kb_update(const BoxRec* __restrict__ rec,
-    const BlockRef* __restrict__ blocks, unsigned ntile, double rhork, double gamrk, int istep,
-    int stats) {
+    const BlockRef* __restrict__ blocks, unsigned ntile, double rhork, double gamrk, int istep) {
   for_tiles<SPAN>(rec, blocks, ntile, [&](const BoxRec* r, const Geom& g, unsigned l) {
-    d_update<R, TP>(g, r->w, fl_prev_of(r, istep), fl_new_of(r, istep), r->sc, rhork, gamrk, istep, stats, r->red,
-                    r->sensor_next, r->sensor, static_cast<R*>(r->aux), Blk{l, 0, 0});
+    d_update<R, TP, MODE>(g, r->w, fl_prev_of(r, istep), fl_new_of(r, istep), r->sc, rhork, gamrk, istep, r->red,
+                          r->sensor_next, r->sensor, static_cast<R*>(r->aux), Blk{l, 0, 0});
   });
 }
 
@@ -278,8 +277,13 @@ cudaError_t batch_stage_impl(const BoxTable& t, const StageArgs& a, cudaStream_t
     ++*nl;
   }
   const Launch U = launch_of(t, BK_UP);
-  kb_update<1, R, TP><<<U.grid(1), UPD_NT, 0, s>>>(t.rec, U.blocks, U.ntile, a.rhork, a.gamrk, a.istep,
-                                                     a.want_stats);
+  auto upd = [&](auto mode) {
+    kb_update<1, R, TP, decltype(mode)::value><<<U.grid(1), UPD_NT, 0, s>>>(t.rec, U.blocks, U.ntile, a.rhork, a.gamrk,
+                                                                         a.istep);
+  };
+  if (a.want_stats) upd(std::integral_constant<int, 2>{});
+  else if (g.force_var) upd(std::integral_constant<int, 1>{});
+  else upd(std::integral_constant<int, 0>{});
   kb_finish_upd<<<nbox, FIN_NT, 0, s>>>(t.rec, a.want_stats, a.add_time);
   *nl += 2;
   return cudaGetLastError();

@@ -79,7 +79,8 @@ constexpr int MT_MAXW = 9, MT_SEG = 2048;
 // 2048 (32 registers, a little spilling in the update pass), for more loads in flight
 // (1024x256x192 boundary layer, ms per step against the allocator's own choice: update 4.24
 // against 5.02 at 60 registers, 4.51 at 1536 threads; aux 3.01 against 3.23; dt 1.12 against
-// 1.27).  The update pass's blocks are 1024 threads (UPD_MINB of them), the others 256.
+// 1.27).  The update pass's blocks are 1024 threads (UPD_MINB of them; 4.63 at 64 registers and one
+// block), the others 256.
 #ifndef UPD_MINB
 #define UPD_MINB 2
 #endif
@@ -581,7 +582,7 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group 
 // boundary layer, ms per step: 16.7 with the stencil loaded by every face into registers, 13.7 read
 // from L1 as often as used, 11.5 from the buffer.
 // fl is written (first contribution of the stage, euler_x after init_flux).
-constexpr int XG_MAX = 8, X_SMEM_MAX = 64 * 1024;
+constexpr int XG_MAX = 8, X_SMEM_MAX = 96 * 1024;  // rows of 4 cells, WENO7 in FP64: 78 KB
 struct XShape {
   int ngrp, slots;
   unsigned nblk;
@@ -1391,17 +1392,19 @@ __global__ void __launch_bounds__(FIN_NT) k_finish_rhs(Geom g, const double* __r
 // update_flux + force_rhs_2 + update_field (kernels_cpu.F90:3400-3442, 3092-3116) and the
 // partials of force_var_1 (:3241-3282) and of compute_residual / minmax (:6682-6810).  All FP64;
 // the primitive values of the stage's starting state are recomputed from w as eval_aux does.
-template <class R, bool TP = false>
+// MODE: 0 the update alone, 1 with the bulk temperature's partials (force_var), 2 with the residual
+// and extrema too (the last stage of a step).  Memory bound (160 bytes a cell) while the registers
+// hold a cell's loads: a pass with what its stage needs only spills 28 to 96 bytes at 32 registers
+// where one for all spilled 48 and loaded w twice (1024x256x192 4.54 -> 4.14 ms per step,
+// 512x256x256 channel 4.14 -> 2.97).  The quotients stay divisions: the series of rcp_pos keeps more
+// values alive (4.93 and 3.56 ms).
+template <class R, bool TP, int MODE>
 __device__ __forceinline__ void d_update(const Geom& g, double* __restrict__ w, const double* __restrict__ fl_prev,
                                                 const double* __restrict__ fl_new, const Scalars* __restrict__ sc,
-                                                double rhork, double gamrk, int istep, int stats,
+                                                double rhork, double gamrk, int istep,
                                                 double* __restrict__ red, const double* __restrict__ sensor_next,
                                                 double* __restrict__ sensor, R* __restrict__ aux, const Blk blk) {
-  constexpr int NW = UPD_NT / 32;
-  __shared__ double sm[2 * NW];
-  __shared__ double smn[3 * NW];
-  __shared__ double smx[3 * NW];
-  double s2[2] = {0.0, 0.0};
+  double sv = 0.0, sr = 0.0;
   double mn[3] = {DBL_MAX, DBL_MAX, DBL_MAX};
   double mx[3] = {-100.0, -100.0, -100.0};
   const long long q = (long long)blk.x * UPD_NT + threadIdx.x;
@@ -1413,68 +1416,77 @@ __device__ __forceinline__ void d_update(const Geom& g, double* __restrict__ w, 
     const double rhodt = rhork * dt, gamdt = gamrk * dt;
     // the stage's starting temperature is in aux (Newton start of the thermally perfect gas)
     const double t_aux = TP ? double(aux[5 * n + c]) : g.t0;
-    const Prim old = prim_from_w<TP>(g, w, c, t_aux);
-    double fln[5];
+    double wo[5], wn[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) wo[m] = w[m * n + c];
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
-      double a = istep > 1 ? -(rhodt * fl_prev[m * nI + q]) : 0.0;
-      fln[m] = a - gamdt * fl_new[m * nI + q];
+      const double a = istep > 1 ? -(rhodt * fl_prev[m * nI + q]) : 0.0;
+      wn[m] = a - gamdt * fl_new[m * nI + q];  // fln
     }
     if (g.channel_case) {
       const double b1 = sc->bulk[0], b2 = sc->bulk[1];
-      fln[0] = fln[0] - b1;
-      fln[1] = fln[1] - b2;
-      fln[4] = fln[4] - old.uu * b2;
+      wn[0] = wn[0] - b1;
+      wn[1] = wn[1] - b2;
+      wn[4] = wn[4] - wo[1] * (1.0 / wo[0]) * b2;
     }
-    double wn[5];
+    const double fln1 = wn[1];
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
-      wn[m] = w[m * n + c] + fln[m];
+      wn[m] = wo[m] + wn[m];
       w[m * n + c] = wn[m];
     }
     // the stage-3 sensor becomes current once every flux of the stage has used the old one
     if (istep == 3) sensor[q] = sensor_next[q];
-    double tstat = old.tt;
-    if (g.force_var) {
-      double dy = g.yn[j + 1] - g.yn[j];
-      double ri = 1.0 / wn[0];
-      double uu = wn[1] * ri, vv = wn[2] * ri, ww = wn[3] * ri;
-      double qq = 0.5 * (uu * uu + vv * vv + ww * ww);
-      double ee = wn[4] / wn[0] - qq;
-      double tt = t_from_e<TP>(g, ee, t_aux);
-      s2[0] = s2[0] + wn[1] * tt * dy;
-      tstat = tt;
+    // temperature of a state
+    auto temp = [&](const double (&s)[5]) {
+      const double ri = 1.0 / s[0];
+      const double uu = s[1] * ri, vv = s[2] * ri, ww = s[3] * ri;
+      return t_from_e<TP>(g, s[4] * ri - 0.5 * (uu * uu + vv * vv + ww * ww), t_aux);
+    };
+    double tt = 0.0;
+    if (MODE >= 1 && g.force_var) {
+      tt = temp(wn);
+      sv = wn[1] * tt * (g.yn[j + 1] - g.yn[j]);
       // force_var_1 leaves this temperature in w_aux(6), where the statistics read it
       if (istep == 3) aux[5 * n + c] = R(tt);
     }
-    if (stats) {
-      double r = fln[1] / dt;
-      s2[1] = s2[1] + r * r;
-      double rho = old.rho;
-      double pp = rho * tstat * g.rgas0;
-      mn[0] = fmin(mn[0], rho); mn[1] = fmin(mn[1], tstat); mn[2] = fmin(mn[2], pp);
-      mx[0] = fmax(mx[0], rho); mx[1] = fmax(mx[1], tstat); mx[2] = fmax(mx[2], pp);
+    if constexpr (MODE == 2) {
+      if (!g.force_var) tt = temp(wo);
+      const double r = fln1 / dt;
+      sr = r * r;
+      const double pp = wo[0] * tt * g.rgas0;
+      mn[0] = mx[0] = wo[0];
+      mn[1] = mx[1] = tt;
+      mn[2] = mx[2] = pp;
     }
   }
-  // the block partials are read only by the forcing and by a stats sample (the same branch for
-  // the whole grid)
-  if (!g.force_var && !stats) return;
+  if constexpr (MODE == 0) return;
+  constexpr int NW = UPD_NT / 32;
+  __shared__ double sm[2 * NW], smn[3 * NW], smx[3 * NW];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* o = red + (long long)blk.x * NRED_UPD;
+  if constexpr (MODE == 1) {
+    double s1[1] = {sv};
+    block_reduce_sum<1, UPD_NT>(s1, sm);
+    if (threadIdx.x == 0) o[0] = s1[0];
+    return;
+  }
+  double s2[2] = {sv, sr};
   block_reduce_sum<2, UPD_NT>(s2, sm);
   // min / max (exact, order independent)
 #pragma unroll
   for (int r = 0; r < 3; ++r)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      mn[r] = fmin(mn[r], __shfl_down_sync(0xffffffffu, mn[r], o));
-      mx[r] = fmax(mx[r], __shfl_down_sync(0xffffffffu, mx[r], o));
+    for (int of = 16; of > 0; of >>= 1) {
+      mn[r] = fmin(mn[r], __shfl_down_sync(0xffffffffu, mn[r], of));
+      mx[r] = fmax(mx[r], __shfl_down_sync(0xffffffffu, mx[r], of));
     }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0)
 #pragma unroll
     for (int r = 0; r < 3; ++r) { smn[r * NW + warp] = mn[r]; smx[r * NW + warp] = mx[r]; }
   __syncthreads();
   if (threadIdx.x == 0) {
-    double* o = red + (long long)blk.x * NRED_UPD;
     o[0] = s2[0];
     o[1] = s2[1];
     for (int r = 0; r < 3; ++r) {
@@ -1485,13 +1497,13 @@ __device__ __forceinline__ void d_update(const Geom& g, double* __restrict__ w, 
     }
   }
 }
-template <class R, bool TP = false>
+template <class R, bool TP, int MODE>
 __global__ void __launch_bounds__(UPD_NT, UPD_MINB) k_update(Geom g, double* __restrict__ w, const double* __restrict__ fl_prev,
                                                 const double* __restrict__ fl_new, const Scalars* __restrict__ sc,
-                                                double rhork, double gamrk, int istep, int stats,
+                                                double rhork, double gamrk, int istep,
                                                 double* __restrict__ red, const double* __restrict__ sensor_next,
                                                 double* __restrict__ sensor, R* __restrict__ aux) {
-  d_update<R, TP>(g, w, fl_prev, fl_new, sc, rhork, gamrk, istep, stats, red, sensor_next, sensor, aux, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
+  d_update<R, TP, MODE>(g, w, fl_prev, fl_new, sc, rhork, gamrk, istep, red, sensor_next, sensor, aux, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
 }
 
 // force_var (singleideal_cpu.F90:890-933): energy shift for the next pass; residual and extrema

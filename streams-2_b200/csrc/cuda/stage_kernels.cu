@@ -291,9 +291,14 @@ static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, do
     ++*nl;
   }
   const unsigned nbu = pt_blocks(g.nint);
-  SB_LAUNCH(d, K_UPDATE, s,
-            k_update<R, (FS & 2) != 0><<<nbu, UPD_NT, 0, s>>>(g, d.w, fl_prev, fl_new, d.sc, a.rhork, a.gamrk, a.istep,
-                                            a.want_stats, d.red, sensor_next, sensor, aux));
+  auto upd = [&](auto mode) {
+    SB_LAUNCH(d, K_UPDATE, s,
+              k_update<R, (FS & 2) != 0, decltype(mode)::value><<<nbu, UPD_NT, 0, s>>>(
+                  g, d.w, fl_prev, fl_new, d.sc, a.rhork, a.gamrk, a.istep, d.red, sensor_next, sensor, aux));
+  };
+  if (a.want_stats) upd(std::integral_constant<int, 2>{});
+  else if (g.force_var) upd(std::integral_constant<int, 1>{});
+  else upd(std::integral_constant<int, 0>{});
   SB_LAUNCH(d, K_FINISH_UPD, s, k_finish_upd<<<1, FIN_NT, 0, s>>>(g, d.red, nbu, a.want_stats, a.add_time, d.sc));
   *nl += 2;
   if (has_stored_ghosts(g)) launch_bc_fill(g, d, s, nl);  // update_ghost

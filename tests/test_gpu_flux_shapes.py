@@ -14,11 +14,11 @@ from conftest import channel_ini, requires_gpu
 pytestmark = [pytest.mark.gpu, requires_gpu]
 
 
-def step_errors(tmp_path, ini, tuning=None, steps=1):
+def step_errors(tmp_path, ini, tuning=None, steps=1, precision=0):
     from oracle_py import Oracle
     from streams_b200 import Case, Solver
     case = Case(tmp_path, ini)
-    s = Solver.from_case(case)
+    s = Solver.from_case(case, precision=precision)
     if tuning:
         s.set_tuning(*tuning)
     s.init_run()
@@ -45,6 +45,17 @@ def test_segments(tmp_path, tuning):
                                 dict(flux_splitting=1), dict(nkeep=2)])
 def test_stencil_widths(tmp_path, kw):
     assert max(step_errors(tmp_path, channel_ini(nx=33, ny=20, nz=19, **kw))) <= 1e-12
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_shortest_rows_with_the_widest_stencil(tmp_path, precision):
+    """Rows of ng cells: the x pass's buffer at its largest."""
+    ini = channel_ini(nx=4, ny=12, nz=5, ep_order=8, weno_scheme=4)
+    if precision == 0:
+        assert max(step_errors(tmp_path, ini)) <= 1e-12
+    else:
+        # FP32 fluxes of one step: a few hundred roundings of 6e-8 on perturbations of a tenth
+        assert max(step_errors(tmp_path, ini, precision=1)) <= 1e-5
 
 
 def test_several_groups_of_faces_and_long_lines(tmp_path):
