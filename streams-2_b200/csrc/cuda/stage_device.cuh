@@ -580,7 +580,7 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group 
 // warp's own buffer while the group before is computed (no block barrier anywhere): 32 points and
 // 2S - 1 more for every row that the group touches, and the sensor beside them.  1024x256x192
 // boundary layer, ms per step: 16.7 with the stencil loaded by every face into registers, 13.7 read
-// from L1 as often as used, 11.5 from the buffer.
+// from L1 as often as used, 11.5 from the buffer (10.7 with the present weno_flux).
 // fl is written (first contribution of the stage, euler_x after init_flux).
 constexpr int XG_MAX = 8, X_SMEM_MAX = 96 * 1024;  // rows of 4 cells, WENO7 in FP64: 78 KB
 struct XShape {
@@ -719,13 +719,14 @@ __global__ void __launch_bounds__(XF_NT, sizeof(R) == 8 ? XF_MINB_D : XF_MINB_F)
 // the address arithmetic and the latency of global loads; the warps' fluxes meet in shared memory,
 // where the cells between them find both faces.  A face is a chain of about a thousand FP64
 // operations, most of them dependent: what bounds the pass is how many are in flight (22 % of the
-// warp slots at 128 registers, FP64 pipe about 55 % in y and 50 % in z).
+// warp slots at 128 registers, FP64 pipe 60 % in y and 54 % in z).
 // Against a thread marching alone along its line with the stencil in registers (168 of them, and
-// 51 KB of scratch per block), 1024x256x192 boundary layer: y 17.0 -> 12.2, z 20.5 -> 13.6 ms per
+// 51 KB of scratch per block), 1024x256x192 boundary layer: y 17.0 -> 11.0, z 20.5 -> 12.5 ms per
 // step; and since a segment takes a round per block of faces instead of a face at a time, a
-// 32x24x16 channel's z pass 93 -> 19 us, its y pass 66 -> 19 us.  What a cell adds to is read before
-// the barrier after the fluxes, which hides it behind the other warps' faces (read after it: y 12.6,
-// z 16.1; copied to shared memory a round ahead: 13.6, 17.3, the copies' own instructions).
+// 32x24x16 channel's z pass 93 -> 17 us, its y pass 66 -> 19 us.  What a cell adds to is read before
+// the barrier after the fluxes, which hides it behind the other warps' faces (in an earlier form:
+// read after it y 12.6, z 16.1; copied to shared memory a round ahead 13.6, 17.3, the copies' own
+// instructions; read before it 12.2, 13.6).
 // The z pass also applies the grad(mu div/3) term of visflx_div_ord2_subroutine
 // (kernels_cpu.F90:3446-3480) and emits the force_rhs block partials (:3157-3193).
 //
@@ -981,7 +982,7 @@ __global__ void __launch_bounds__(sizeof(R) == 8 ? MT_MAXT_D : MT_MAXT_F, 1) k_m
 // of the context: of the divisions of a cell (6 by face distances, 6 by the Prandtl number, one by
 // 3) none is left.
 // 1024x256x192 boundary layer, FP64: 7.4 -> 4.2 ms per step (its 112 algorithmic bytes a cell take
-// 2.5 at the copy rate); 1024x256x128 mixed: 3.4 -> 1.96; a 32x24x16 channel, whose segments were
+// 2.5 at the copy rate); 1024x256x128 mixed: 3.4 -> 2.1; a 32x24x16 channel, whose segments were
 // 16 cells: 57 -> 9 us a pass.
 constexpr int VT_X = 32, VT_Y = 8, VT_NT = VT_X * VT_Y, VT_KMAX = 16;
 constexpr int VT_PX = VT_X + 2, VT_PY = VT_Y + 2, VT_PP = VT_PX * VT_PY;
