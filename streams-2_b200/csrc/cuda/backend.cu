@@ -243,7 +243,11 @@ void fill_geom(streams_b200_ctx* c) {
     g.rpr = 1.0 / p.prandtl;
     g.weps_a = 0.000001 * r2u2;
     g.weps_b = 0.000001 * r2u4;
-    g.weps_c = 0.000001 * r2u6;
+    auto pow2_near_reciprocal = [](double x) { return std::isnormal(x) ? std::ldexp(1.0, -std::ilogb(x)) : 1.0; };
+    g.wzs_b = pow2_near_reciprocal(r2u4);
+    g.wsc_c = pow2_near_reciprocal(p.rho0 * u0_2 * p.u0);
+    g.wsr_c = 1.0 / g.wsc_c;
+    g.weps_c = 0.000001 * r2u6 * g.wsc_c * g.wsc_c;
     g.wbs_a = 1.0 / r2u2;
     g.wbs_b = 1.0 / r2u4;
     g.wbs_c = g.wbs_b / u0_2;

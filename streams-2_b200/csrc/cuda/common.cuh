@@ -88,6 +88,10 @@ struct Geom {
   // 1/(rho0^2 u0^4) of wenorec_1d (kernels_cpu.F90:2539-2546) and 1/(rho0^2 u0^6), and its 1e-6 over
   // each of them
   double gm1, rgm1, rcp0, rcv0, rt0, cpp, rpr, wbs_a, wbs_b, wbs_c, weps_a, weps_b, weps_c;
+  // powers of two by which weno_rec's products stay in the exponent range in slow flows: next to the
+  // indicator scale 1/(rho0^2 u0^4); next to 1/(rho0 u0^3), for an energy flux itself (weps_c is of the
+  // flux scaled by it), and its reciprocal
+  double wzs_b, wsc_c, wsr_c;
   // thermally perfect gas (calorically_perfect = 0): cp(T) = sum of cpc[l - cp_l] (T/t0)^l for
   // l = cp_l..cp_r, cv likewise (set_fluid_prop's cp_coeff / cv_coeff, times rgas0)
   int calorically_perfect, cp_l, cp_r;

@@ -291,8 +291,8 @@ __device__ __forceinline__ float wenorec(const float (&vp)[2 * WS], const float 
 // otherwise a lower one, ord, next to a boundary (chosen at run time in every side, 1024x256x192:
 // 49.0 -> 48.1 ms per step; y and z spill 4 and 28 bytes for 40 and 48).
 template <int WS, bool WZ, bool FULL>
-__device__ __forceinline__ void weno_side(const double (&v)[2 * WS - 1], int ord, double eps2, double& base, double& num,
-                                          double& den) {
+__device__ __forceinline__ void weno_side(const double (&v)[2 * WS - 1], int ord, double eps2, double zs, double& base,
+                                          double& num, double& den) {
   using R = double;
   constexpr int c = WS - 1;
   base = v[c];
@@ -317,14 +317,14 @@ __device__ __forceinline__ void weno_side(const double (&v)[2 * WS - 1], int ord
         n2 = p01 * p01;
       } else {
         // WENO-Z, omega_k = d_k (beta_k + tau)/(beta_k + eps); eps is a single-precision literal in
-        // the reference
-        const R eps = R(4.0 * static_cast<double>(1.e-35f) / 0.000001) * eps2;
+        // the reference.  The factors are scaled by zs where they are summed, which costs and rounds nothing.
+        const R eps = R(4.0 * static_cast<double>(1.e-35f) / 0.000001) * eps2 * zs;
         const R e0 = b0 * b0 + (k * s0) * s0, e1 = b1 * b1 + (k * s1) * s1, e2 = b2 * b2 + (k * s2) * s2;
-        const R tau = fabs(e0 - e2) + eps;
-        const R f0 = e0 + eps, f1 = e1 + eps, f2 = e2 + eps;
-        n0 = (e0 + tau) * (f1 * f2);
-        n1 = R(6) * ((e1 + tau) * (f0 * f2));
-        n2 = (e2 + tau) * (f0 * f1);
+        const R tau = fma(fabs(e0 - e2), zs, eps);
+        const R f0 = fma(e0, zs, eps), f1 = fma(e1, zs, eps), f2 = fma(e2, zs, eps);
+        n0 = fma(e0, zs, tau) * (f1 * f2);
+        n1 = R(6) * (fma(e1, zs, tau) * (f0 * f2));
+        n2 = fma(e2, zs, tau) * (f0 * f1);
       }
       // sum of the weights (n2's factor 3 apart), and of the candidates less base = v[c] + d1/2, which
       // are s0/3, s1/3 and s1/2 - s2/6
@@ -370,14 +370,18 @@ __device__ __forceinline__ void weno_side(const double (&v)[2 * WS - 1], int ord
   }
 }
 // wenorec_1d of one variable in FP64: the two sides of the face, p in upwind order from the left, m
-// from the right, with one reciprocal for both (the denominators are positive and stay far inside the
-// exponent range).
+// from the right, with one reciprocal for both.  The product of the denominators must stay above 2.2e-308
+// where neither side has differences: it is then 100 e^8 for WENO-JS, e = 4 eps2, and 100 e^6 for WENO-Z,
+// e = 4e-29 eps2 zs.  With eps2 = 1e-6 rho0^2 u0^2 (the mass flux, entropy and acoustic fields; rho0 = 1)
+// that holds for u0 above 3e-9; with u0^4 (momentum fluxes, shear fields) it holds for WENO-JS above 5e-9,
+// and for WENO-Z by the power of two zs next to 1/(rho0^2 u0^4) (without it above 5e-5 only); an energy
+// flux (u0^6) comes scaled to order 1 by a power of two (else above 3e-6 and 1.4e-3 only).
 template <int WS, bool WZ, bool FULL>
 __device__ __forceinline__ double weno_rec(const double (&p)[2 * WS - 1], const double (&m)[2 * WS - 1], int ord,
-                                           double eps2) {
+                                           double eps2, double zs) {
   double bp, np, dp, bm, nm, dm;
-  weno_side<WS, WZ, FULL>(p, ord, eps2, bp, np, dp);
-  weno_side<WS, WZ, FULL>(m, ord, eps2, bm, nm, dm);
+  weno_side<WS, WZ, FULL>(p, ord, eps2, zs, bp, np, dp);
+  weno_side<WS, WZ, FULL>(m, ord, eps2, zs, bm, nm, dm);
   return (bp + bm) + (np * dm + nm * dp) * rcp_pos(dp * dm);
 }
 
@@ -642,7 +646,7 @@ __device__ __forceinline__ void weno_flux(const Geom& g, const LN& ln, int ord, 
       if (l < 2 * WS - 1) gp[l] = T + ev1 * P;
       if (l > 0) gm[2 * WS - 1 - l] = T - ev1 * P;
     }
-    fi[2 + m] = weno_rec<WS, WZ, FULL>(gp, gm, ord, g.weps_b * 4.0) * 0.5;
+    fi[2 + m] = weno_rec<WS, WZ, FULL>(gp, gm, ord, g.weps_b * 4.0, g.wzs_b) * 0.5;
   }
   // the entropy field, and P_m(U) and T_m = P_m(F) of the two acoustic ones (g+- = T +- lambda P)
   const R epsa = g.weps_a;
@@ -667,7 +671,7 @@ __device__ __forceinline__ void weno_flux(const Geom& g, const LN& ln, int ord, 
       if (l < 2 * WS - 1) gp[l] = T + ev1 * E;
       if (l > 0) gm[2 * WS - 1 - l] = T - ev1 * E;
     }
-    fi[1] = weno_rec<WS, WZ, FULL>(gp, gm, ord, epsa * 4.0) * 0.5;
+    fi[1] = weno_rec<WS, WZ, FULL>(gp, gm, ord, epsa * 4.0, 1.0) * 0.5;
   }
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
@@ -679,7 +683,7 @@ __device__ __forceinline__ void weno_flux(const Geom& g, const LN& ln, int ord, 
       if (l < 2 * WS - 1) gp[l] = T + lam * P;
       if (l > 0) gm[2 * WS - 1 - l] = T - lam * P;
     }
-    fi[4 * m] = weno_rec<WS, WZ, FULL>(gp, gm, ord, epsa * 16.0) * 0.25;
+    fi[4 * m] = weno_rec<WS, WZ, FULL>(gp, gm, ord, epsa * 16.0, 1.0) * 0.25;
   }
   // back-projection with the right eigenvectors, er(m,:) = (1, u - c n, h - vn c) for m = 1,
   // (1, u, b3) for m = 2, (0, e_t, v_t) for m = 3, 4, (1, u + c n, h + vn c) for m = 5
@@ -844,8 +848,13 @@ __device__ __forceinline__ void rusanov_flux(const Geom& g, const LN& ln, int or
         evm = rhou;
         c = R(0.5) * (evm + rhoevm);
       } else if (m == 4) {
-        evm = h * rhou;
-        c = R(0.5) * (evm + evmax * (rho * h - pp));
+        R hs = h, ps = pp;
+        if constexpr (sizeof(R) == sizeof(double)) {  // scaled for weno_rec
+          hs = g.wsc_c * h;
+          ps = g.wsc_c * pp;
+        }
+        evm = hs * rhou;
+        c = R(0.5) * (evm + evmax * (rho * hs - ps));
       } else {
         const R vd = m == 1 ? vel[0] : (m == 2 ? vel[1] : vel[2]);
         evm = vd * rhou;
@@ -863,7 +872,9 @@ __device__ __forceinline__ void rusanov_flux(const Geom& g, const LN& ln, int or
         p[l] = gp[l];
         q[l] = gm[2 * WS - 1 - l];
       }
-      v = weno_rec<WS, WZ, FULL>(p, q, ord, m == 0 ? g.weps_a : (m == 4 ? g.weps_c : g.weps_b));
+      v = weno_rec<WS, WZ, FULL>(p, q, ord, m == 0 ? g.weps_a : (m == 4 ? g.weps_c : g.weps_b),
+                                 m == 0 || m == 4 ? 1.0 : g.wzs_b);
+      if (m == 4) v = v * g.wsr_c;
     } else {
       v = wenorec<WS>(gp, gm, ord, WZ ? 1 : 0, m == 0 ? R(g.wbs_a) : (m == 4 ? R(g.wbs_c) : R(g.wbs_b)));
     }
