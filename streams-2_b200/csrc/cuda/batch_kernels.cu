@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(AUX_NT, DT ? AUX_MINB_DT : AUX_MINB) kb_aux(co
 }
 
 template <unsigned SPAN, class R, int LB, int WS, int FS>
-__global__ void __launch_bounds__(XF_NT, sizeof(R) == 8 ? XF_MINB_D : XF_MINB_F)
+__global__ void __launch_bounds__(XF_NT, x_minb<R, LB, FS>())
     kb_xflux(const BoxRec* __restrict__ rec, const BlockRef* __restrict__ blocks, unsigned ntile, int istep) {
   for_tiles<SPAN>(rec, blocks, ntile, [&](const BoxRec* r, const Geom& g, unsigned l) {
     d_xflux<R, LB, WS, FS>(g, static_cast<const R*>(r->aux), r->sensor, fl_new_of(r, istep), r->xgrp, Blk{l, 0, 0});
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256) kb_sensor(const BoxRec* __restrict__ rec,
 }
 
 template <unsigned SPAN, class R, int DIR, int LB, int WS, bool CH, int FS>
-__global__ void __launch_bounds__(sizeof(R) == 8 ? MT_MAXT_D : MT_MAXT_F, 1)
+__global__ void __launch_bounds__(march_maxt<R, LB, FS>(), 1)
     kb_march(const BoxRec* __restrict__ rec, const BlockRef* __restrict__ blocks, unsigned ntile, double rhork, double gamrk, int istep) {
   for_tiles<SPAN>(rec, blocks, ntile, [&](const BoxRec* r, const Geom& g, unsigned l) {
     const int seglen = DIR == 1 ? r->sly : r->slz, nseg = DIR == 1 ? r->nsy : r->nsz;

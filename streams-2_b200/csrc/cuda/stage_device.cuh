@@ -61,6 +61,16 @@ constexpr int MT_MAXW = 9, MT_SEG = 2048;
 #ifndef WF_MINB_D
 #define WF_MINB_D 3
 #endif
+// KEEP(n) (FS & 4) of order 8 in FP64, whose central flux holds eight values of eight points, takes 168
+// registers: at 128 its passes spill up to 576 bytes (256x128x128 channel in noise, WENO7, ms per step
+// for nkeep = -1, 1, 2: 15.0, 20.0, 25.1 at 128; 13.1, 18.6, 21.6 at 168; a marching form of 168
+// registers 14.5, 21.3, 23.5).  Order 6 stays at 128: nkeep = 2 10.0 against 10.3 at 168.
+template <class R, int LB, int FS>
+constexpr bool wide_keep() { return sizeof(R) == sizeof(double) && LB == 4 && (FS & 4) != 0; }
+template <class R, int LB, int FS>
+constexpr int x_minb() { return sizeof(R) == sizeof(float) ? XF_MINB_F : (wide_keep<R, LB, FS>() ? 3 : XF_MINB_D); }
+template <class R, int LB, int FS>
+constexpr int march_maxt() { return sizeof(R) == sizeof(float) ? MT_MAXT_F : (wide_keep<R, LB, FS>() ? 384 : MT_MAXT_D); }
 #ifndef WF_MINB_F
 #define WF_MINB_F 4
 #endif
@@ -707,7 +717,7 @@ __device__ __forceinline__ void d_xflux(const Geom& g, const R* __restrict__ aux
   }
 }
 template <class R, int LB, int WS, int FS = 0>
-__global__ void __launch_bounds__(XF_NT, sizeof(R) == 8 ? XF_MINB_D : XF_MINB_F)
+__global__ void __launch_bounds__(XF_NT, x_minb<R, LB, FS>())
     k_xflux(Geom g, const R* __restrict__ aux, const double* __restrict__ sensor, double* __restrict__ fl, int ngrp) {
   d_xflux<R, LB, WS, FS>(g, aux, sensor, fl, ngrp, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
 }
@@ -961,7 +971,7 @@ __device__ __forceinline__ void d_march(const Geom& g, const R* __restrict__ aux
   }
 }
 template <class R, int DIR, int LB, int WS, bool CH = false, int FS = 0, bool SPLIT = false>
-__global__ void __launch_bounds__(sizeof(R) == 8 ? MT_MAXT_D : MT_MAXT_F, 1) k_march(Geom g, const R* __restrict__ aux,
+__global__ void __launch_bounds__(march_maxt<R, LB, FS>(), 1) k_march(Geom g, const R* __restrict__ aux,
                                                  const double* __restrict__ sensor, double* __restrict__ fl,
                                                  const R* __restrict__ div3,
                                                  const double* __restrict__ w, const double* __restrict__ fl_prev,

@@ -42,7 +42,8 @@ def test_segments(tmp_path, tuning):
 
 
 @pytest.mark.parametrize("kw", [dict(ep_order=8, weno_scheme=4), dict(ep_order=4, weno_scheme=2), dict(weno_version=1),
-                                dict(flux_splitting=1), dict(nkeep=2)])
+                                dict(flux_splitting=1), dict(nkeep=2), dict(ep_order=8, weno_scheme=4, nkeep=-1),
+                                dict(ep_order=8, weno_scheme=4, nkeep=2)])
 def test_stencil_widths(tmp_path, kw):
     assert max(step_errors(tmp_path, channel_ini(nx=33, ny=20, nz=19, **kw))) <= 1e-12
 
