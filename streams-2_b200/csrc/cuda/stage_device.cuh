@@ -1524,13 +1524,15 @@ __device__ __forceinline__ void d_finish_upd(const Geom& g, const double* __rest
   __shared__ double smn[3 * (FIN_NT / 32)], smx[3 * (FIN_NT / 32)];
   double v[2] = {0.0, 0.0};
   double mn[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, mx[3] = {-100.0, -100.0, -100.0};
-  // k_update wrote block partials only for the forcing or a stats sample
+  // k_update wrote all block partials for a stats sample, the first alone for the forcing, else none
   const long long nb = (g.force_var || stats) ? nblk : 0;
   for (long long b = threadIdx.x; b < nb; b += FIN_NT) {
     const double* o = red + b * NRED_UPD;
     v[0] = v[0] + o[0];
-    v[1] = v[1] + o[1];
-    for (int r = 0; r < 3; ++r) { mn[r] = fmin(mn[r], o[2 + r]); mx[r] = fmax(mx[r], o[5 + r]); }
+    if (stats) {
+      v[1] = v[1] + o[1];
+      for (int r = 0; r < 3; ++r) { mn[r] = fmin(mn[r], o[2 + r]); mx[r] = fmax(mx[r], o[5 + r]); }
+    }
   }
   block_reduce_sum<2, FIN_NT>(v, sm);
 #pragma unroll
