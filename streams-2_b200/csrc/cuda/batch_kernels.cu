@@ -149,10 +149,10 @@ template <unsigned SPAN, class R, int DIR, int LB, int WS, bool CH, int FS>
 __global__ void __launch_bounds__(march_maxt<R, LB, FS>(), 1)
     kb_march(const BoxRec* __restrict__ rec, const BlockRef* __restrict__ blocks, unsigned ntile, double rhork, double gamrk, int istep) {
   for_tiles<SPAN>(rec, blocks, ntile, [&](const BoxRec* r, const Geom& g, unsigned l) {
-    const int seglen = DIR == 1 ? r->sly : r->slz, nseg = DIR == 1 ? r->nsy : r->nsz;
+    const int seglen = DIR == 1 ? r->sly : r->slz;
     d_march<R, DIR, LB, WS, CH, FS, false>(g, static_cast<const R*>(r->aux), r->sensor, fl_new_of(r, istep),
                                            static_cast<const R*>(r->div3), r->w, fl_prev_of(r, istep), r->sc, rhork,
-                                           gamrk, istep, seglen, nseg, r->red, Blk{l, 0, 0});
+                                           gamrk, istep, seglen, r->red, Blk{l, 0, 0});
   });
 }
 
@@ -363,8 +363,8 @@ BoxRec box_rec(const Geom& g, const DevState& d, double* fl_a, double* fl_b, dou
   r.sc = d.sc;
   r.cfl = cfl;
   const MarchShape my = march_shape(g, 1), mz = march_shape(g, 2);
-  r.sly = my.seglen; r.nsy = my.nseg;
-  r.slz = mz.seglen; r.nsz = mz.nseg;
+  r.sly = my.seglen;
+  r.slz = mz.seglen;
   r.nwy = my.nwarps; r.nwz = mz.nwarps;
   const XShape xs = x_shape(g);
   r.nb_x = xs.nblk;

@@ -14,40 +14,38 @@
 
 namespace sb200 {
 
-// Quotient and square root (of a positive value) in the flux arithmetic: IEEE in FP64, where the
-// reference's operations are kept; with SB_FP32_FAST the FP32 form takes the hardware reciprocal
-// and reciprocal square root (at most 2 ulp: the mixed form's error is set by FP32 rounding).
+// Quotient and square root (of a positive value) of the mixed form's FP32 flux arithmetic: with
+// SB_FP32_FAST the hardware reciprocal and reciprocal square root (at most 2 ulp: the form's error is
+// set by FP32 rounding) instead of the IEEE routines.
 // With SB_FP32_FAST = 2 the approximate reciprocal r of b is refined by one Newton-Raphson step
 // (e = 1 - b r, r += r e) and the quotient q = a r corrected by its remainder (Markstein:
 // q += r (a - b q)); the approximate reciprocal square root y of x gives s = x y, corrected by one
 // Newton step for the square root (s += (x - s s) y / 2).  Without the refinement the errors of
 // the raw approximations do not average out over many steps (the transverse momenta of a
 // WENO-only channel drifted twice as far from the FP64 oracle in 100 steps).
-template <class R>
-__device__ __forceinline__ R fdiv(R a, R b) {
-  if constexpr (sizeof(R) == sizeof(double) || !SB_FP32_FAST) {
-    return a / b;
-  } else if constexpr (SB_FP32_FAST == 1) {
-    return __fdividef(a, b);
-  } else {
-    float r = __fdividef(1.0f, b);
-    const float e = __fmaf_rn(-b, r, 1.0f);
-    r = __fmaf_rn(r, e, r);
-    const float q = a * r;
-    return __fmaf_rn(r, __fmaf_rn(-b, q, a), q);
-  }
+__device__ __forceinline__ float fdiv(float a, float b) {
+#if !SB_FP32_FAST
+  return a / b;
+#elif SB_FP32_FAST == 1
+  return __fdividef(a, b);
+#else
+  float r = __fdividef(1.0f, b);
+  const float e = __fmaf_rn(-b, r, 1.0f);
+  r = __fmaf_rn(r, e, r);
+  const float q = a * r;
+  return __fmaf_rn(r, __fmaf_rn(-b, q, a), q);
+#endif
 }
-template <class R>
-__device__ __forceinline__ R fsqrt_pos(R x) {
-  if constexpr (sizeof(R) == sizeof(double) || !SB_FP32_FAST) {
-    return sqrt(x);
-  } else if constexpr (SB_FP32_FAST == 1) {
-    return x * rsqrtf(x);
-  } else {
-    const float y = rsqrtf(x);
-    const float sx = x * y;
-    return __fmaf_rn(__fmaf_rn(-sx, sx, x), 0.5f * y, sx);
-  }
+__device__ __forceinline__ float fsqrt_pos(float x) {
+#if !SB_FP32_FAST
+  return sqrtf(x);
+#elif SB_FP32_FAST == 1
+  return x * rsqrtf(x);
+#else
+  const float y = rsqrtf(x);
+  const float sx = x * y;
+  return __fmaf_rn(__fmaf_rn(-sx, sx, x), 0.5f * y, sx);
+#endif
 }
 
 // maximum that keeps b when a is not a number (as fmax does for the running maxima here), without

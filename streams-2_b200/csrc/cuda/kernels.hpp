@@ -136,7 +136,7 @@ struct BoxRec {
   double* red;
   Scalars* sc;
   double cfl;
-  int sly, nsy, slz, nsz;  // march segments (length, count) of the y and z passes
+  int sly, slz;            // segment lengths of the y and z passes
   int nwy, nwz;            // and the warps of their blocks
   int xgrp, vk;            // x pass: groups of 32 faces a warp takes; viscous pass: cells of a z segment
   unsigned nb_x, nb_vol, nb_pt, nb_y, nb_z;  // blocks of the aux pass, pointwise passes, y and z passes

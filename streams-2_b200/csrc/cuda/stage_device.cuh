@@ -544,7 +544,7 @@ template <class R, int DIR, int LB, int WS, int S, int FS, class LN>
 __device__ __forceinline__ void weno_face(const Geom& g, const LN& ln, int ep, double (&f)[5], const Scr<R>& scr) {
   const int ord = max(WS + ep, 1);
   auto flux = [&](auto full) {
-    constexpr bool FULL = decltype(full)::value;
+    [[maybe_unused]] constexpr bool FULL = decltype(full)::value;
     if constexpr ((FS & 1) != 0) rusanov_flux<R, DIR, WS, S, (FS & 2) != 0, (FS & 8) != 0, FULL>(g, ln, ord, f);
     else if constexpr (sizeof(R) == sizeof(double)) weno_flux<DIR, WS, S, (FS & 2) != 0, (FS & 8) != 0, FULL>(g, ln, ord, f, scr);
     else weno_flux_f<DIR, WS, S, (FS & 8) != 0>(g, ln, ord, f, scr);
@@ -758,7 +758,7 @@ __device__ __forceinline__ void d_march(const Geom& g, const R* __restrict__ aux
                                                  const R* __restrict__ div3,
                                                  const double* __restrict__ w, const double* __restrict__ fl_prev,
                                                  const Scalars* __restrict__ sc, double rhork, double gamrk,
-                                                 int istep, int seglen, int nseg, double* __restrict__ red, const Blk blk) {
+                                                 int istep, int seglen, double* __restrict__ red, const Blk blk) {
   static_assert(DIR == 1 || DIR == 2, "march kernel handles y and z");
   constexpr int S = LB > WS ? LB : WS;
   extern __shared__ __align__(16) unsigned char sb_dyn_smem[];
@@ -976,8 +976,8 @@ __global__ void __launch_bounds__(march_maxt<R, LB, FS>(), 1) k_march(Geom g, co
                                                  const R* __restrict__ div3,
                                                  const double* __restrict__ w, const double* __restrict__ fl_prev,
                                                  const Scalars* __restrict__ sc, double rhork, double gamrk,
-                                                 int istep, int seglen, int nseg, double* __restrict__ red) {
-  d_march<R, DIR, LB, WS, CH, FS, SPLIT>(g, aux, sensor, fl, div3, w, fl_prev, sc, rhork, gamrk, istep, seglen, nseg, red, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
+                                                 int istep, int seglen, double* __restrict__ red) {
+  d_march<R, DIR, LB, WS, CH, FS, SPLIT>(g, aux, sensor, fl, div3, w, fl_prev, sc, rhork, gamrk, istep, seglen, red, Blk{blockIdx.x, blockIdx.y, blockIdx.z});
 }
 
 // The viscous pass: visflx_reduced_ord2_subroutine (kernels_cpu.F90:4623-4721, update_sensor = 0)
@@ -1776,7 +1776,7 @@ inline XShape x_shape(const Geom& g) {
   return x;
 }
 
-// Launch shape of a y or z pass: segments of seglen cells (nseg of them on each line) and the warps
+// Launch shape of a y or z pass: segments of seglen cells of a line and the warps
 // of a block.  The segments are at least minseg cells and at most as many as bring the pass to
 // about target threads; among the counts allowed, the one with the least estimated time is taken:
 // rounds of a segment's seglen + 1 faces over the block's warps times the blocks an SM works
@@ -1785,13 +1785,13 @@ inline XShape x_shape(const Geom& g) {
 // (a function of the box alone, so that a box has the same partition in every form it runs in).
 constexpr int LW = 4, MT_FREE = 4;
 struct MarchShape {
-  int seglen, nseg, nwarps;
+  int seglen, nwarps;
   unsigned nblk;
 };
 inline MarchShape march_shape_with(const Geom& g, int dir, long long target, int minseg) {
   const int emin = dir == 1 ? g.eul_jmin : g.eul_kmin, emax = dir == 1 ? g.eul_jmax : g.eul_kmax;
   const int ncell = emax - emin + 1;
-  if (ncell < 1) return MarchShape{1, 0, LW, 0};
+  if (ncell < 1) return MarchShape{1, LW, 0};
   const long long lines = (long long)g.nx * (dir == 1 ? g.nz : g.ny);
   const long long tiles = (lines + 31) / 32;
   const long long most = std::min<long long>(std::max(1, ncell / minseg), (target + lines * LW - 1) / (lines * LW));
@@ -1811,8 +1811,7 @@ inline MarchShape march_shape_with(const Geom& g, int dir, long long target, int
   }
   MarchShape m;
   m.seglen = (ncell + bn - 1) / bn;
-  m.nseg = (ncell + m.seglen - 1) / m.seglen;
-  const long long blocks = tiles * m.nseg;
+  const long long blocks = tiles * ((ncell + m.seglen - 1) / m.seglen);
   m.nblk = (unsigned)blocks;
   const int room = (int)std::min<long long>(MT_MAXW, 148LL * MT_MAXW / std::max<long long>(1, blocks));
   m.nwarps = LW;

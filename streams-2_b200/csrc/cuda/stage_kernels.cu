@@ -252,11 +252,11 @@ static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, do
   if (my.nblk > 0) {
     SB_LAUNCH(d, K_EULER_Y, s,
               k_march<R, 1, LB, WS, false, FS><<<my.nblk, 32 * my.nwarps, ysm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev, d.sc,
-                                                          a.rhork, a.gamrk, a.istep, my.seglen, my.nseg, d.red));
+                                                          a.rhork, a.gamrk, a.istep, my.seglen, d.red));
     if (split_on) {
       SB_LAUNCH(d, K_EULER_Y, s,
                 k_march<R, 1, LB, WS, false, FS, true><<<my.nblk, 32 * my.nwarps, yss, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
-                                                                   d.sc, a.rhork, a.gamrk, a.istep, my.seglen, my.nseg, d.red));
+                                                                   d.sc, a.rhork, a.gamrk, a.istep, my.seglen, d.red));
       ++*nl;
     }
   }
@@ -268,19 +268,19 @@ static cudaError_t stage_impl(const Geom& g, DevState& d, const StageArgs& a, do
   if (g.channel_case) {
     SB_LAUNCH(d, K_EULER_Z, s,
               k_march<R, 2, LB, WS, true, FS><<<mz.nblk, 32 * mz.nwarps, zsm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev, d.sc,
-                                                                  a.rhork, a.gamrk, a.istep, mz.seglen, mz.nseg, d.red));
+                                                                  a.rhork, a.gamrk, a.istep, mz.seglen, d.red));
     if (split_on)
       SB_LAUNCH(d, K_EULER_Z, s,
                 k_march<R, 2, LB, WS, true, FS, true><<<mz.nblk, 32 * mz.nwarps, zss, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
-                                                                  d.sc, a.rhork, a.gamrk, a.istep, mz.seglen, mz.nseg, d.red));
+                                                                  d.sc, a.rhork, a.gamrk, a.istep, mz.seglen, d.red));
   } else {
     SB_LAUNCH(d, K_EULER_Z, s,
               k_march<R, 2, LB, WS, false, FS><<<mz.nblk, 32 * mz.nwarps, zsm, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev, d.sc,
-                                                                   a.rhork, a.gamrk, a.istep, mz.seglen, mz.nseg, d.red));
+                                                                   a.rhork, a.gamrk, a.istep, mz.seglen, d.red));
     if (split_on)
       SB_LAUNCH(d, K_EULER_Z, s,
                 k_march<R, 2, LB, WS, false, FS, true><<<mz.nblk, 32 * mz.nwarps, zss, s>>>(g, aux, sensor, fl_new, div3, d.w, fl_prev,
-                                                                   d.sc, a.rhork, a.gamrk, a.istep, mz.seglen, mz.nseg, d.red));
+                                                                   d.sc, a.rhork, a.gamrk, a.istep, mz.seglen, d.red));
   }
   if (split_on) ++*nl;
   *nl += 4;
