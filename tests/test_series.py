@@ -1,6 +1,7 @@
 """The series by which the device refines its approximate reciprocal and reciprocal square root
 (rcp_pos, rsqrt_pos): with any start of 20 correct bits the result is within 1.5 units in the last
-place, every operation rounded to double as the device rounds it (fused multiply-adds once)."""
+place, every operation rounded to double as the device rounds it (fused multiply-adds once).  This is
+the derivation of the bound; test_gpu_reciprocals.py measures the device functions against it."""
 import math
 import random
 from fractions import Fraction as Q
