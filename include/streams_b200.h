@@ -17,7 +17,7 @@
  *   - A context owns all of its device memory and one CUDA stream.  Calls on one context
  *     are not reentrant; distinct contexts may be driven from distinct host threads.
  *   - The device path computes in FP64 (precision = 0) or in the mixed form (precision = 1:
- *     FP32 flux and viscous arithmetic with compensated flux-difference sums; FP64 state,
+ *     FP32 flux and viscous arithmetic, face fluxes summed and differenced in FP64; FP64 state,
  *     RK register, temperature recovery and reductions).
  */
 #ifndef STREAMS_B200_H
@@ -303,7 +303,8 @@ int streams_b200_get_tuning(streams_b200_ctx* ctx, long long* march_threads, int
  * within the fraction.  1 always computes the WENO faces apart; 0 turns the split off (the hybrid
  * passes alone, no list or face kernel launched).  Default: 0.55 for boxes of at least 2^21
  * cells, 0 for smaller ones (launch-bound, where the split's extra launches cost more than it
- * saves).  The face buffers (about 53 bytes per cell) are allocated when the split is first on;
+ * saves).  In FP64 the hybrid passes are as fast or faster with their WENO faces at every fraction
+ * measured (0), in the mixed form the split is ahead below about 0.4.  The face buffers (about 53 bytes per cell) are allocated when the split is first on;
  * STREAMS_B200_ENOMEM if that fails.  Both forms evaluate the same arithmetic: FP64 results are
  * identical up to the compiler's contraction of the WENO arithmetic in the two kernels
  * (observed: bit-identical, or differences of a few ulp).

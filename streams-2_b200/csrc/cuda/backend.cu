@@ -89,14 +89,21 @@ cudaError_t dev_alloc(streams_b200_ctx* c, T** p, size_t count) {
 }
 
 // Largest WENO face fraction of a direction at which its hybrid pass reads the WENO faces from
-// the face buffer: measured on the 1024x256x192 boundary layer, the split form is ahead below a
-// fraction of about 0.55 (FP64: 85.2 vs 87.0 ms per step at 0.51, 89.0 vs 87.3 at 0.61; 61.9 vs
-// 78.1 at 0.06) and behind above it (99.8 vs 86.8 at 0.90).
+// the face buffer, as the interface states it: the break-even of hybrid passes that marched along
+// lines (FP64, 1024x256x192 boundary layer: 85.2 apart against 87.0 ms per step inside at 0.51, 89.0
+// against 87.3 at 0.61).  With the present passes, ms per step inside / apart at fractions of
+//          0.01       0.08       0.13       0.35       0.55       0.75
+//   FP64   32.2/32.9  36.9/38.8  41.7/45.7  46.4/54.8  47.5/61.5  47.6/67.6
+//   mixed  28.4/28.1  34.1/32.7  39.7/37.3  44.6/43.2  45.7/47.7  45.8/52.1
+// (512x256x256 channel at 0.05, 0.25, 0.50: FP64 27.7/27.7, 32.0/36.5, 32.9/40.6; mixed 27.0/25.1,
+// 31.6/30.3, 32.5/33.0): inside is the better form in FP64 at every fraction, apart in the mixed form
+// below about 0.4.  A caller's set_weno_split overrides the default.
 constexpr double WENO_SPLIT_FRAC_DEFAULT = 0.55;
 // Boxes below this many cells start with the split off (fraction 0: the hybrid passes alone, no
 // list or face kernels launched and no buffers held).  A small box's step is launch-bound and the
 // split adds about twenty launches per step, most of them leaving at once; measured on the
-// served channel boxes of 0.13 - 1.2 M cells: 501 -> 436 Mcell-steps/s with the split on.
+// served channel boxes of 0.13 - 1.2 M cells, with the marching passes: 501 -> 436 Mcell-steps/s
+// with the split on.
 constexpr long long WENO_SPLIT_MIN_CELLS = 1LL << 21;
 
 long long footprint(const streams_b200_params* p) {
@@ -122,7 +129,7 @@ long long footprint(const streams_b200_params* p) {
 
 std::string validate(const streams_b200_params* p) {
   if (p->nx < 1 || p->ny < 1 || p->nz < 1) return "grid sizes must be positive";
-  // the x pass's launch grid carries ny / 4 rows in its y and nz planes in its z dimension
+  // limits of the interface (launch grids carry rows and planes in their y and z dimensions)
   if (p->ny > 4 * 65535 || p->nz > 65535) return "ny must be at most 262140 and nz at most 65535";
   if (p->ep_order < 2 || p->ep_order > 8 || p->ep_order % 2) return "ep_order must be 2, 4, 6 or 8";
   const int lmax = p->ep_order / 2;
@@ -285,7 +292,7 @@ cudaError_t ensure_weno_buffers(streams_b200_ctx* c) {
     return e;
   g.wbits = wb;
   g.wface = wf;
-  g.nwface = nfmax;  // plane stride: 5 planes of doubles, or 10 planes of floats in the same bytes
+  g.nwface = nfmax;  // stride of the 5 planes
   g.wlist[0] = wl;
   g.wlist[1] = wl + nfx;
   g.wlist[2] = wl + nfx + nfy;

@@ -177,7 +177,7 @@ struct Scalars {
 // last place.  Arguments are positive and normal (densities, squared sound speeds, sums of weights).
 // They stand for the IEEE quotients and square roots, which branch for their special cases, of the
 // Roe average (three) and of the weights (one for the two sides of a field) of a WENO face, and for
-// the quotients by the density of the pointwise passes.
+// the quotients by the density of the aux, time-step and energy-shift passes.
 __device__ __forceinline__ double rcp_pos(double b) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));

@@ -276,18 +276,18 @@ __device__ __forceinline__ float wenorec(const float (&vp)[2 * WS], const float 
   return R(0);
 }
 
-// One side of wenorec_1d (kernels_cpu.F90:2526-2724): v[0 .. 2WS-2] in upwind order (the upwind
-// cell of the face at v[WS-1]) eps2 = 1e-6 over the
-// reference's scale of the smoothness indicators.  The side's value is base + num/den.
+// One side of wenorec_1d (kernels_cpu.F90:2526-2724): v[0 .. 2WS-2] in upwind order (the upwind cell
+// of the face at v[WS-1]), eps2 = 1e-6 over the reference's scale of the smoothness indicators, zs as
+// weno_rec says.  The side's value is base + num/den.
 // The indicators and candidates are written in first and second differences d, s of the points:
 // beta_k = 13/12 s_k^2 + 1/4 b_k^2 with b_k = 3 d - d', d + d', d' - 3 d, and the candidates share
 // the upwind cell and d1/2; the weights' common factors (1/4 of the indicators, 1/10 of the weights)
 // cancel.  With the projection of weno_flux a face of the FP64 y pass executes 880 FP64 instructions
 // (central faces of its warp included) where the point values, with the fluxes projected beside the
 // states and IEEE quotients, took 1415.
-// FULL: order WS, in straight-line code that the two sides and the fields share the schedule of;
-// otherwise a lower one, ord, next to a boundary (chosen at run time in every side, 1024x256x192:
-// 49.0 -> 48.1 ms per step; y and z spill 4 and 28 bytes for 40 and 48).
+// FULL: order WS, in straight-line code that the two sides and the fields share the schedule of
+// (1024x256x192, ms per step: 48.1 against 49.0 with the order chosen at run time in every side);
+// otherwise a lower one, ord, next to a boundary.
 template <int WS, bool WZ, bool FULL>
 __device__ __forceinline__ void weno_side(const double (&v)[2 * WS - 1], int ord, double eps2, double zs, double& base,
                                           double& num, double& den) {

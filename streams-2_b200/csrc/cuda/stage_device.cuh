@@ -35,7 +35,7 @@ namespace sb200 {
 namespace {
 
 constexpr int AUX_NT = 256;
-constexpr int XF_TX = 32, XF_TY = 4, XF_NT = XF_TX * XF_TY;  // x faces: 4 row-warps per block
+constexpr int XF_TX = 32, XF_TY = 4, XF_NT = XF_TX * XF_TY;  // x faces: 4 warps per block
 // y / z passes: blocks of LW = 4 warps, up to MT_MAXW in small boxes; segments of at most MT_SEG cells
 constexpr int MT_MAXW = 9, MT_SEG = 2048;
 // Registers of the flux kernels, as the threads an SM shall hold (y / z: 65536 / MT_MAXT_* registers
@@ -480,14 +480,13 @@ __device__ __forceinline__ int face_ep(const Geom& g, int p) {
 // WENO faces apart (1) or always inside the hybrid passes (0).  Apart, the faces whose stencil
 // sees the sensor are listed per direction once per step and computed by their own kernel at
 // full occupancy; the hybrid passes read their fluxes from a face buffer.  A warp of the hybrid
-// passes otherwise runs both branches whenever one of its faces is a WENO face, which with
-// scattered WENO faces costs nearly a full WENO pass.  When most faces are WENO faces the
-// buffer's extra traffic and the stencil loads without the passes' sliding window cost more
-// than that, so each direction chooses on the device from its list's length (weno_split): the
-// x pass holds both branches, the y and z passes are launched in both forms and the one not
-// chosen leaves at once (about a thousand blocks; the x pass's grid is too large for that).
-// The lists themselves are built only when a sample of every 16th plane is within the
-// threshold, so a step that keeps its WENO faces in the hybrid passes pays for the sample only.
+// passes otherwise runs both branches whenever one of its faces is a WENO face.  The face kernels
+// gather their stencils one sector a value and the buffer is written and read, so each direction
+// chooses on the device from its list's length (weno_split): the x pass holds both branches, the y
+// and z passes are launched in both forms and the one not chosen leaves at once.  The lists
+// themselves are built only when a sample of every 16th plane is within the threshold, so a step
+// that keeps its WENO faces in the hybrid passes pays for the sample and the unused launches
+// (0.3 of 47.6 ms per step at 1024x256x192).  What either form costs: WENO_SPLIT_FRAC_DEFAULT.
 #ifndef SB_WENO_SPLIT
 #define SB_WENO_SPLIT 1
 #endif
@@ -999,7 +998,7 @@ constexpr int VT_PX = VT_X + 2, VT_PY = VT_Y + 2, VT_PP = VT_PX * VT_PY;
 template <class R>
 constexpr size_t visc_smem() { return (size_t)VT_NT * 4 * 8 + (size_t)4 * 5 * VT_PP * sizeof(R); }
 // blocks: 32 x 8 columns x segments of vk cells in z, VT_KMAX of them (two more planes are loaded per
-// segment) or fewer where that leaves SMs without their three blocks
+// segment) or as few as give each SM three blocks (two are resident in FP64, four in FP32)
 inline int visc_k(const Geom& g) {
   const long long tiles = (long long)((g.nx + VT_X - 1) / VT_X) * ((g.ny + VT_Y - 1) / VT_Y);
   return (int)std::min<long long>(VT_KMAX, std::max<long long>(1, tiles * g.nz / (148 * 3)));
@@ -1405,9 +1404,9 @@ __global__ void __launch_bounds__(FIN_NT) k_finish_rhs(Geom g, const double* __r
 // the primitive values of the stage's starting state are recomputed from w as eval_aux does.
 // MODE: 0 the update alone, 1 with the bulk temperature's partials (force_var), 2 with the residual
 // and extrema too (the last stage of a step).  Memory bound (160 bytes a cell) while the registers
-// hold a cell's loads: a pass with what its stage needs only spills 28 to 96 bytes at 32 registers
-// where one for all spilled 48 and loaded w twice (1024x256x192 4.54 -> 4.14 ms per step,
-// 512x256x256 channel 4.14 -> 2.97).  The quotients stay divisions: the series of rcp_pos keeps more
+// hold a cell's loads: a pass with what its stage needs only spills 8, 28 and 44 bytes (MODE 0, 1, 2; the
+// thermally perfect gas 8, 108 and 284) at 32 registers where one for all spilled 48 and loaded w twice
+// (1024x256x192 4.54 -> 4.14 ms per step, 512x256x256 channel 4.14 -> 2.97).  The quotients stay divisions: the series of rcp_pos keeps more
 // values alive (4.93 and 3.56 ms).
 template <class R, bool TP, int MODE>
 __device__ __forceinline__ void d_update(const Geom& g, double* __restrict__ w, const double* __restrict__ fl_prev,
